@@ -30,6 +30,7 @@
 
 #include <cmath>
 
+#include "binomial_filter.hpp"
 #include "common.hpp"
 #include "math.hpp"
 #include "random.hpp"
@@ -153,6 +154,39 @@ DUST2_HD bool binomial_n_ok(std::uint64_t nb) {
   return nb < 0x7ff0000000000000ull || nb == BITS_MINUS_ZERO;
 }
 
+// Binomial(n, pp) for a valid n > 0 and pp in (0, 1/2], in FP64.
+DUST2_SAMPLER double binomial_fp64(rng_state& rng, double n, double pp) {
+  const double q = 1.0 - pp;
+  // n * pp < 10 (n * pp is positive and finite)
+  if (math::bits_of(n * pp) < BITS_TEN) {
+    const double s = pp * math::rcp(q);
+    return binomial_inversion(rng, n, pp, q, s, math::log(q));
+  }
+  return binomial_btrs(rng, n, pp, q, math::quiet_nan());
+}
+
+#if defined(__CUDA_ARCH__)
+// On the device a draw is first decided in FP32 (binomial_filter.hpp); an
+// undecided one (some in 10^4), a count that is not an integer below 2^24
+// and a probability below 2^-60 take the FP64 sampler.  That one works on
+// a copy of the generator, so that the kernel's own stays in registers.
+__device__ __forceinline__ double binomial_decided(rng_state& rng, double n,
+                                                   double pp,
+                                                   const filter::prob& f) {
+  float nf;
+  if (filter::count_of(n, &nf) && math::bits_of(pp) >= filter::BITS_MIN_P) {
+    const int k = filter::binomial(rng, n, pp, nf, f);
+    if (k >= 0) {
+      return filter::count_to_double(k);
+    }
+  }
+  rng_state r = rng;
+  const double x = binomial_fp64(r, n, pp);
+  rng = r;
+  return x;
+}
+#endif
+
 // Binomial(n, p) for integer-valued n >= 0 and p in [0, 1].  The argument
 // checks are taken on the bit patterns, with the FP64 semantics of
 // !(n >= 0) || !finite(n) || !(p >= 0) || !(p <= 1) (so -0 is valid).
@@ -175,15 +209,11 @@ DUST2_HD double binomial(rng_state& rng, double n, double p) {
   }
   const bool flip = pb > BITS_HALF;  // p > 1/2
   const double pp = flip ? 1.0 - p : p;
-  const double q = 1.0 - pp;
-  // n * pp < 10 (n * pp is positive and finite)
-  double x;
-  if (math::bits_of(n * pp) < BITS_TEN) {
-    const double s = pp * math::rcp(q);
-    x = binomial_inversion(rng, n, pp, q, s, math::log(q));
-  } else {
-    x = binomial_btrs(rng, n, pp, q, math::quiet_nan());
-  }
+#if defined(__CUDA_ARCH__)
+  const double x = binomial_decided(rng, n, pp, filter::make_prob(pp));
+#else
+  const double x = binomial_fp64(rng, n, pp);
+#endif
   return flip ? n - x : x;
 }
 
@@ -202,6 +232,7 @@ struct binomial_prob {
   std::uint64_t bits;
   bool valid;
   bool flip;
+  filter::prob f;  // pp, as the device's FP32 decisions take it
 };
 
 DUST2_HD binomial_prob binomial_prepare(double p) {
@@ -212,10 +243,14 @@ DUST2_HD binomial_prob binomial_prepare(double p) {
   b.flip = b.valid && b.bits > BITS_HALF;
   b.pp = b.flip ? 1.0 - p : p;
   if (b.valid && (b.bits << 1) != 0 && b.bits != BITS_ONE) {
+#if defined(__CUDA_ARCH__)
+    b.f = filter::make_prob(b.pp);
+#else
     b.q = 1.0 - b.pp;
     b.s = b.pp * math::rcp(b.q);
     b.logq = math::log(b.q);
     b.lpq = math::log(b.s);
+#endif
   }
   return b;
 }
@@ -235,12 +270,16 @@ DUST2_HD double binomial(rng_state& rng, double n, const binomial_prob& b) {
   if (b.bits == BITS_ONE) {
     return n;
   }
+#if defined(__CUDA_ARCH__)
+  const double x = binomial_decided(rng, n, b.pp, b.f);
+#else
   double x;
   if (math::bits_of(n * b.pp) < BITS_TEN) {
     x = binomial_inversion(rng, n, b.pp, b.q, b.s, b.logq);
   } else {
     x = binomial_btrs(rng, n, b.pp, b.q, b.lpq);
   }
+#endif
   return b.flip ? n - x : x;
 }
 
