@@ -175,8 +175,9 @@ __device__ __forceinline__ double binomial_decided(rng_state& rng, double n,
                                                    const filter::prob& f) {
   float nf;
   if (filter::count_of(n, &nf) && math::bits_of(pp) >= filter::BITS_MIN_P) {
-    const int k = filter::binomial(rng, n, pp, nf, f);
-    if (k >= 0) {
+    const float k =
+      filter::binomial(rng, nf, f, [&] { return n * pp < 10.0 ? 1 : 0; });
+    if (k >= 0.0f) {
       return filter::count_to_double(k);
     }
   }

@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "common.hpp"
+#include "count_draws.hpp"
 #include "distributions.hpp"
 #include "math.hpp"
 #include "random.hpp"
@@ -187,6 +188,43 @@ struct has_update<T, std::void_t<decltype(&T::update)>> : std::true_type {};
 template <typename T>
 constexpr bool is_continuous() {
   return has_rhs<T>::value;
+}
+
+// Count stepping (device only): a system whose state entries are counts
+// may declare
+//   count_update(time, dt, float* c, shared, rng): one update in place, on
+//     the state as FP32 counts, returning exactly what update() does;
+//   count_fits(const float* c): whether every entry stays below
+//     random::COUNT_LIMIT whatever the draws;
+//   count_prepare(shared_state&, dt) (host): fills shared.counts, whose
+//     member `ready(dt)` says whether the group can be stepped this way.
+// A particle whose entries are not all counts, or that does not fit, is
+// stepped by update().
+template <class T, class = void>
+struct has_count_update : std::false_type {};
+template <class T>
+struct has_count_update<T, std::void_t<decltype(&T::count_update)>>
+  : std::true_type {};
+
+// The shared state as a kernel sees it: with the count tables of `dt`.
+template <typename T>
+void prepare_counts(typename T::shared_state& shared, double dt) {
+  if constexpr (has_count_update<T>::value) {
+    T::count_prepare(shared, dt);
+  } else {
+    (void)shared;
+    (void)dt;
+  }
+}
+
+// Bytes of those tables.
+template <typename T>
+constexpr std::size_t count_table_bytes() {
+  if constexpr (has_count_update<T>::value) {
+    return sizeof(T::shared_state::counts);
+  } else {
+    return 0;
+  }
 }
 
 // Mixed time: an ODE (rhs) with a discrete-time update applied every dt

@@ -129,11 +129,12 @@ __device__ __forceinline__ void store_state(const system_view<T>& v, int k,
 }
 
 // Reset the zero_every entries due at step `step` (time `time`): the
-// first ZERO_STEPS_CACHED steps read the block's precomputed masks.
-template <typename T>
+// first ZERO_STEPS_CACHED steps read the block's precomputed masks.  The
+// state is doubles, or FP32 counts.
+template <typename T, typename R>
 __device__ __forceinline__ void apply_zero_every(
     const zero_every_spec& z, const std::uint64_t* zero_steps, int step,
-    double time, double* x) {
+    double time, R* x) {
   for (int i = 0; i < z.n; ++i) {
     const bool hit = (zero_steps != nullptr && step < ZERO_STEPS_CACHED) ?
       ((zero_steps[i] >> step) & 1) != 0 : fmod(time, z.period[i]) == 0;
@@ -205,6 +206,84 @@ __device__ __forceinline__ void run_particle(
       }
     }
   }
+}
+
+// Advance particle k n_steps by update() from its state in device memory,
+// and store it again: out of line, for the few particles of a system with
+// count_update that cannot be stepped as counts.
+template <typename T>
+__device__ __noinline__ void step_particle_update(
+    const system_view<T>& v, int k, double time, double dt, int n_steps,
+    const typename T::shared_state& shared, const zero_every_spec& z,
+    const std::uint64_t* zero_steps, random::rng_state& rng) {
+  typename T::internal_state internal{};
+  double x[T::n_state_max];
+  double y[update_in_place_of<T>::value ? 1 : T::n_state_max];
+  load_state<T>(v, k, x);
+  run_particle<T>(time, dt, n_steps, shared, internal, z, zero_steps, rng, x,
+                  y);
+  store_state<T>(v, k, x);
+}
+
+// Advance particle k n_steps from its state in device memory and store
+// it again; then done(x, internal) runs on the new state.  Systems with
+// count_update step a particle whose state is counts in FP32
+// (dust2gpu/count_draws.hpp), without an FP64 instruction and with half
+// the registers or local memory; the entries go from memory to FP32 and
+// back by their bits.
+template <typename T, typename F>
+__device__ __forceinline__ void step_particle(
+    const system_view<T>& v, int k, double time, double dt, int n_steps,
+    const typename T::shared_state& shared, const zero_every_spec& z,
+    const std::uint64_t* zero_steps, random::rng_state& rng, const F& done) {
+  typename T::internal_state internal{};
+  double x[T::n_state_max];
+  if constexpr (has_count_update<T>::value) {
+    float c[T::n_state_max];
+    bool ok = !v.deterministic && shared.counts.ready(dt);
+    if (ok) {
+#pragma unroll
+      for (int s = 0; s < T::n_state_max; ++s) {
+        c[s] = 0;
+        if (s < v.n_state) {
+          ok &= random::filter::count_of(
+            v.state[static_cast<long>(s) * v.stride + k], &c[s]);
+        }
+      }
+      ok = ok && T::count_fits(c);
+    }
+    if (ok) {
+      for (int i = 0; i < n_steps; ++i) {
+        const double t = time + static_cast<double>(i) * dt;
+        apply_zero_every<T>(z, zero_steps, i, t, c);
+        T::count_update(t, dt, c, shared, rng);
+      }
+#pragma unroll
+      for (int s = 0; s < T::n_state_max; ++s) {
+        if (s < v.n_state) {
+          x[s] = random::filter::count_to_double(c[s]);
+          v.state[static_cast<long>(s) * v.stride + k] = x[s];
+        }
+      }
+    } else {
+      random::rng_state r = rng;
+      step_particle_update<T>(v, k, time, dt, n_steps, shared, z, zero_steps,
+                              r);
+      rng = r;
+      load_state<T>(v, k, x);
+    }
+    if constexpr (T::n_state_max > 32) {
+      // too large for registers: `done` reads what it needs from memory
+      load_state<T>(v, k, x);
+    }
+  } else {
+    double y[update_in_place_of<T>::value ? 1 : T::n_state_max];
+    load_state<T>(v, k, x);
+    run_particle<T>(time, dt, n_steps, shared, internal, z, zero_steps, rng,
+                    x, y);
+    store_state<T>(v, k, x);
+  }
+  done(x, internal);
 }
 
 // Pick a block size for a system: big states need more registers per
@@ -308,13 +387,9 @@ DUST2_PARTICLE_KERNEL(T) k_run(system_view<T> v, double time, double dt,
   const auto& shared = mixed ? v.shared[g] : sm.shared();
   const zero_every_spec& zero = mixed ? v.zero_every[g] : sm.zero;
   auto rng = load_rng(v.rng, v.stride, k, v.deterministic);
-  typename T::internal_state internal{};
-  double x[T::n_state_max];
-  double y[update_in_place_of<T>::value ? 1 : T::n_state_max];
-  load_state<T>(v, k, x);
-  run_particle<T>(time, dt, n_steps, shared, internal, zero,
-                  mixed ? nullptr : sm.zero_steps, rng, x, y);
-  store_state<T>(v, k, x);
+  step_particle<T>(v, k, time, dt, n_steps, shared, zero,
+                   mixed ? nullptr : sm.zero_steps, rng,
+                   [](const double*, typename T::internal_state&) {});
   store_rng(v.rng, v.stride, k, rng);
   capture_error(v.errors, v.any_error, k, rng);
 }
@@ -766,6 +841,9 @@ public:
   }
 
   void upload_shared() {
+    for (auto& s : shared_) {
+      prepare_counts<T>(s, dt_);
+    }
     DUST2_CUDA(cudaMemcpyAsync(shared_dev_.data(), shared_.data(),
                                shared_.size() * sizeof(shared_state),
                                cudaMemcpyHostToDevice, stream_));

@@ -158,14 +158,12 @@ __device__ __forceinline__ void step_compare_tile(
   if (valid) {
     const int k = tl.start + threadIdx.x;
     auto rng = load_rng(v.rng, v.stride, k, v.deterministic);
-    typename T::internal_state internal{};
-    double x[T::n_state_max];
-    double y[update_in_place_of<T>::value ? 1 : T::n_state_max];
-    load_state<T>(v, k, x);
-    run_particle<T>(time, dt, n_steps, sm.shared(), internal, sm.zero,
-                    sm.zero_steps, rng, x, y);
-    logw = T::compare_data(time_compare, x, *d, sm.shared(), internal, rng);
-    store_state<T>(v, k, x);
+    step_particle<T>(v, k, time, dt, n_steps, sm.shared(), sm.zero,
+                     sm.zero_steps, rng,
+                     [&](const double* x, typename T::internal_state& in) {
+                       logw = T::compare_data(time_compare, x, *d,
+                                              sm.shared(), in, rng);
+                     });
     store_rng(v.rng, v.stride, k, rng);
     capture_error(v.errors, v.any_error, k, rng);
     f.w[k] = logw;

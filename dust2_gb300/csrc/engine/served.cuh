@@ -297,12 +297,14 @@ public:
     }
     DUST2_CUDA(cudaGetDevice(&device_));
     // memory plan: 1/16 of the budget for data and schedules, the rest
-    // for particles
+    // for particles (the slots' count tables, about 1 KB each, come on
+    // top)
     const double per_obs = sizeof(data_type) + sizeof(obs_step);
     long n_obs_cap = static_cast<long>(hbm_budget_bytes / 16 / per_obs);
     n_obs_cap = std::max(1024L, std::min(n_obs_cap, 1L << 26));
     const double slot_bytes = static_cast<double>(n_slots_) *
-      (sizeof(shared_state) + sizeof(zero_every_spec) + 256);
+      (sizeof(shared_state) - count_table_bytes<T>() +
+       sizeof(zero_every_spec) + 256);
     double left = hbm_budget_bytes - n_obs_cap * per_obs - slot_bytes;
     long n_cap = static_cast<long>(left / bytes_per_particle());
     n_cap = std::min(n_cap, 1L << 29) / ALIGN * ALIGN;
@@ -447,6 +449,7 @@ public:
     auto ss = std::make_unique<session>();
     ss->n = n_particles;
     ss->shared = T::build_shared(pars);
+    prepare_counts<T>(ss->shared, dt);
     ss->dt = dt;
     ss->time_start = time_start;
     double t = time_start;
@@ -486,6 +489,7 @@ public:
       // update_pars semantics (r/filter.hpp:101-110): constants kept
       shared_state sh = ss.has_latest ? ss.shared_latest : ss.shared;
       T::update_shared(pars, sh);
+      prepare_counts<T>(sh, ss.dt);
       ss.shared_latest = sh;
       ss.has_latest = true;
     }

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "../dust2gpu/system.hpp"
+#include "sir_counts.hpp"
 
 namespace dust2gpu {
 namespace systems {
@@ -19,6 +20,7 @@ struct sir {
     real_type beta;
     real_type gamma;
     real_type exp_noise;
+    sir_counts counts;
   };
   struct internal_state {};
   struct data_type {
@@ -40,7 +42,7 @@ struct sir {
   static constexpr const char* data_names[] = {"incidence"};
 
   static shared_state build_shared(const double* pars) {
-    shared_state s;
+    shared_state s{};
     s.I0 = read_par<sir>(pars, 0);
     s.N = read_par<sir>(pars, 1);
     s.beta = read_par<sir>(pars, 2);
@@ -111,6 +113,28 @@ struct sir {
     state_next[2] = R + n_IR;
     state_next[3] = cases_cumul + n_SI;
     state_next[4] = cases_inc + n_SI;
+  }
+
+  static void count_prepare(shared_state& s, real_type dt) {
+    s.counts.prepare(s.N, s.beta, s.gamma, dt);
+  }
+
+  // c: S, I, R, cases_cumul, cases_inc (the last two grow by what leaves S)
+  DUST2_HD static bool count_fits(const float* c) {
+    return c[0] + c[1] + c[2] + c[3] + c[4] < random::COUNT_LIMIT;
+  }
+
+  DUST2_HD static void count_update(real_type time, real_type dt, float* c,
+                                    const shared_state& shared,
+                                    rng_state_type& rng_state) {
+    float n_SI, n_IR;
+    shared.counts.draw(rng_state, c[0], c[1], shared.N, shared.beta, dt,
+                       &n_SI, &n_IR);
+    c[0] = c[0] - n_SI;
+    c[1] = c[1] + n_SI - n_IR;
+    c[2] = c[2] + n_IR;
+    c[3] = c[3] + n_SI;
+    c[4] = c[4] + n_SI;
   }
 
   DUST2_HD static real_type compare_data(const real_type time,

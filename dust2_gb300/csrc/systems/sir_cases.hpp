@@ -7,6 +7,7 @@
 #pragma once
 
 #include "../dust2gpu/system.hpp"
+#include "sir_counts.hpp"
 
 namespace dust2gpu {
 namespace systems {
@@ -21,6 +22,7 @@ struct sir_cases {
     real_type I0;
     real_type beta;
     real_type gamma;
+    sir_counts counts;
   };
   // Per-thread scratch (dust2's internal_state): the recovery
   // probability 1 - exp(-gamma dt) and the terms of its binomial draws
@@ -49,7 +51,7 @@ struct sir_cases {
   static constexpr const char* data_names[] = {"incidence"};
 
   static shared_state build_shared(const double* pars) {
-    shared_state s;
+    shared_state s{};
     s.I0 = read_par<sir_cases>(pars, 0);
     s.N = read_par<sir_cases>(pars, 1);
     s.beta = read_par<sir_cases>(pars, 2);
@@ -118,6 +120,28 @@ struct sir_cases {
     state_next[1] = I + n_SI - n_IR;
     state_next[2] = R + n_IR;
     state_next[3] = cases_inc + n_SI;
+  }
+
+  static void count_prepare(shared_state& s, real_type dt) {
+    s.counts.prepare(s.N, s.beta, s.gamma, dt);
+  }
+
+  // c: S, I, R, cases_inc.  S + I + R is constant, and cases_inc grows by
+  // what leaves S.
+  DUST2_HD static bool count_fits(const float* c) {
+    return c[0] + c[1] + c[2] + c[3] < random::COUNT_LIMIT;
+  }
+
+  DUST2_HD static void count_update(real_type time, real_type dt, float* c,
+                                    const shared_state& shared,
+                                    rng_state_type& rng_state) {
+    float n_SI, n_IR;
+    shared.counts.draw(rng_state, c[0], c[1], shared.N, shared.beta, dt,
+                       &n_SI, &n_IR);
+    c[0] = c[0] - n_SI;
+    c[1] = c[1] + n_SI - n_IR;
+    c[2] = c[2] + n_IR;
+    c[3] = c[3] + n_SI;
   }
 
   DUST2_HD static real_type compare_data(const real_type time,

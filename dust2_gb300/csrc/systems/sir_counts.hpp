@@ -1,0 +1,56 @@
+// The two transitions of the SIR systems between FP32 counts
+// (dust2gpu/count_draws.hpp): n_SI ~ Bin(S, 1 - exp(-beta I / N dt)) and
+// n_IR ~ Bin(I, 1 - exp(-gamma dt)), drawn in that order.
+#pragma once
+
+#include <cmath>
+
+#include "../dust2gpu/system.hpp"
+
+namespace dust2gpu {
+namespace systems {
+
+struct sir_counts {
+  std::uint64_t key_dt;
+  std::uint64_t rate62;  // beta dt / N in units of 2^-62: 2^-32 relative
+  random::count_prob recover;
+  bool ok;
+
+  void prepare(double N, double beta, double gamma, double dt) {
+    key_dt = math::bits_of(dt);
+    const double rate = beta * dt / N;
+    recover = random::make_count_prob(1 - math::exp(-gamma * dt));
+    ok = recover.ok && N > 0 && rate >= 0x1p-30 && rate < 1;
+    rate62 = ok ? static_cast<std::uint64_t>(std::ldexp(rate, 62)) : 0;
+  }
+
+  DUST2_HD bool ready(double dt) const {
+    return ok && key_dt == math::bits_of(dt);
+  }
+
+  // I < 2^24 and rate < 1: a hazard of 2 or more would wrap, so it is
+  // bounded in FP32 first (any hazard of 1/2 or more takes the FP64
+  // probability).
+  DUST2_HD void draw(random::rng_state& rng, float S, float I, double N,
+                     double beta, double dt, float* n_SI,
+                     float* n_IR) const {
+    *n_SI = 0;
+    if (I > 0.0f) {
+      const std::uint32_t rate_hi = static_cast<std::uint32_t>(rate62 >> 38);
+      const std::uint64_t x62 =
+        I * (static_cast<float>(rate_hi) + 1.0f) < 0x1p24f ?
+        static_cast<std::uint32_t>(I) * rate62 : ~0ull;
+      *n_SI = random::binomial_hazard(rng, S, x62, 0.0f, [&] {
+        return 1 - math::exp(-beta * filter_to_double(I) / N * dt);
+      });
+    }
+    *n_IR = random::binomial_count(rng, I, recover);
+  }
+
+  DUST2_HD static double filter_to_double(float x) {
+    return random::filter::count_to_double(x);
+  }
+};
+
+}  // namespace systems
+}  // namespace dust2gpu

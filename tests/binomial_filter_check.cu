@@ -36,18 +36,18 @@ DUST2_HD void check(random::rng_state& rng, double n, double p, int n_draws,
     random::rng_state a = rng;
     t.draws++;
     float nf;
-    int k = -1;
+    float k = -1.0f;
     if (random::filter::count_of(n, &nf)) {
-      k = random::filter::binomial(a, n, pp, nf,
-                                   random::filter::make_prob(pp));
+      k = random::filter::binomial(a, nf, random::filter::make_prob(pp),
+                                   [&] { return n * pp < 10.0 ? 1 : 0; });
     }
     random::rng_state b = rng;
     const double want = random::binomial_fp64(b, n, pp);
-    if (k < 0) {
+    if (k < 0.0f) {
       t.undecided++;
       // the FP64 sampler takes over from where the filter stopped
       const double x = random::binomial_fp64(a, n, pp);
-      k = static_cast<int>(x);
+      k = static_cast<float>(x);
     }
     bool same = static_cast<double>(k) == want &&
       math::bits_of(random::filter::count_to_double(k)) ==
