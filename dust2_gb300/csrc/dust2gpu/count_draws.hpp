@@ -38,42 +38,55 @@ DUST2_HD float binomial_count_fp64(rng_state& rng, float n, double p) {
   return static_cast<float>(x);
 }
 
+// The probability of one draw: decided draws use q; where q is not usable
+// the draw takes the FP64 probability at once.
+struct draw_prob {
+  filter::prob q;  // min(p, 1 - p)
+  bool usable;
+  bool zero;       // p is 0
+  bool flip;       // p > 1/2
+};
+
 // A probability that is the same for every particle of a group, made on
 // the host.
 struct count_prob {
-  filter::prob q;  // min(p, 1 - p)
+  draw_prob d;
   double p;
-  double pp;
-  bool zero;
-  bool flip;
-  bool ok;  // usable by binomial_count
+  bool ok;
 };
 
 inline count_prob make_count_prob(double p) {
   count_prob c{};
   c.p = p;
-  c.zero = p == 0;
-  c.flip = p > 0.5;
-  c.pp = c.flip ? 1.0 - p : p;
-  c.ok = c.zero || (p < 1 && c.pp >= 0x1p-60);
-  if (c.ok && !c.zero) {
-    c.q = filter::make_prob(c.pp);
+  c.d.zero = p == 0;
+  c.d.flip = p > 0.5;
+  const double pp = c.d.flip ? 1.0 - p : p;
+  c.d.usable = p < 1 && pp >= 0x1p-60;
+  c.ok = c.d.zero || c.d.usable;
+  if (c.d.usable) {
+    c.d.q = filter::make_prob(pp);
   }
   return c;
 }
 
-// binomial(rng, n, c.p) for a count n.
-DUST2_HD float binomial_count(rng_state& rng, float n, const count_prob& c) {
-  if (n == 0.0f || c.zero) {
+// binomial(rng, n, exact()) for a count n and its probability d.  A system
+// with several draws per step makes them in a loop over one call of this:
+// the sampler is a few hundred instructions, and one copy of it left SEIR
+// at 5 blocks per SM without spilling around it (three copies 75.9 ms).
+template <typename F>
+DUST2_HD float draw_count(rng_state& rng, float n, const draw_prob& d,
+                          const F& exact) {
+  if (n == 0.0f || d.zero) {
     return 0.0f;
   }
-  const float k = filter::binomial(rng, n, c.q, [&] {
-    return filter::count_to_double(n) * c.pp < 10.0 ? 1 : 0;
-  });
-  if (k < 0.0f) {
-    return binomial_count_fp64(rng, n, c.p);
+  if (d.usable) {
+    // n p too close to 10 to choose the sampler: undecided
+    const float k = filter::binomial(rng, n, d.q, [] { return -1; });
+    if (k >= 0.0f) {
+      return d.flip ? n - k : k;
+    }
   }
-  return c.flip ? n - k : k;
+  return binomial_count_fp64(rng, n, exact());
 }
 
 DUST2_HD std::uint32_t mul_hi32(std::uint32_t a, std::uint32_t b) {
@@ -114,21 +127,16 @@ DUST2_HD filter::prob hazard_prob(std::uint64_t x62, float rel) {
   return q;
 }
 
-// binomial(rng, n, exact()) for a count n, where exact() is the FP64
-// evaluation of 1 - exp(-x) and x is within (rel x) of x62 2^-62.  (FP64's
-// own rounding of the probability, 2^-53 absolute, moves n p by less than
-// 2^-29.)  A hazard outside [2^-40, 1/2) takes the FP64 probability.
-template <typename F>
-DUST2_HD float binomial_hazard(rng_state& rng, float n, std::uint64_t x62,
-                               float rel, const F& exact) {
-  if (n == 0.0f) {
-    return 0.0f;
-  }
-  float k = -1.0f;
-  if (x62 - (1ull << 22) < (1ull << 61) - (1ull << 22)) {
-    k = filter::binomial(rng, n, hazard_prob(x62, rel), [] { return -1; });
-  }
-  return k < 0.0f ? binomial_count_fp64(rng, n, exact()) : k;
+// 1 - exp(-x), x within (rel x) of x62 2^-62.  (FP64's own rounding of the
+// probability, 2^-53 absolute, moves n p by less than 2^-29.)  A hazard
+// outside [2^-40, 1/2) is not usable.
+DUST2_HD draw_prob hazard_draw(std::uint64_t x62, float rel) {
+  draw_prob d;
+  d.usable = x62 - (1ull << 22) < (1ull << 61) - (1ull << 22);
+  d.zero = false;
+  d.flip = false;
+  d.q = hazard_prob(x62, rel);
+  return d;
 }
 
 }  // namespace random

@@ -237,6 +237,31 @@ DUST2_HD double u53_to_unit(std::uint64_t m) {
   return from_bits((expo << 52) | mant);
 }
 
+// std::fmod(t, period) == 0, on the bits for a period that is a power of
+// two (the usual daily reset has period 1): t is then a multiple when its
+// lowest set bit is no lower than the period's.
+DUST2_HD bool is_multiple(double t, double period) {
+  const std::uint64_t pb = bits_of(period);
+  const std::uint64_t tb = bits_of(t) & 0x7fffffffffffffffull;
+  const int pe = static_cast<int>(pb >> 52);
+  const int te = static_cast<int>(tb >> 52);
+  if ((pb & 0x000fffffffffffffull) == 0 && pe >= 1 && pe <= 2046 &&
+      (tb == 0 || (te >= 1 && te <= 2046))) {
+    if (tb == 0) {
+      return true;
+    }
+    const std::uint64_t m = (tb & 0x000fffffffffffffull) |
+      0x0010000000000000ull;
+#if defined(__CUDA_ARCH__)
+    const int low = __ffsll(static_cast<long long>(m)) - 1;
+#else
+    const int low = __builtin_ctzll(m);
+#endif
+    return te - 52 + low >= pe;
+  }
+  return std::fmod(t, period) == 0;
+}
+
 // |x| below this (704) takes the fast path of exp: the result is normal
 // and the scaling by 2^e is an exponent add.
 constexpr std::uint64_t EXP_FAST_BITS = 0x4086000000000000ull;
@@ -502,6 +527,13 @@ DUST2_HD std::uint32_t float_bits_of(float x) {
   std::memcpy(&u, &x, sizeof(u));
   return u;
 #endif
+}
+
+// The same value as a double, on the bits, for a normal positive x.
+DUST2_HD double float_to_double(float x) {
+  const std::uint32_t f = float_bits_of(x);
+  return from_bits((static_cast<std::uint64_t>((f >> 3) + 0x38000000u)
+                    << 32) | static_cast<std::uint32_t>(f << 29));
 }
 
 // 1/y for finite y with |y| in [1e-30, 1e30] (within 1 ulp; not

@@ -192,19 +192,62 @@ constexpr bool is_continuous() {
 
 // Count stepping (device only): a system whose state entries are counts
 // may declare
-//   count_update(time, dt, float* c, shared, rng): one update in place, on
-//     the state as FP32 counts, returning exactly what update() does;
-//   count_fits(const float* c): whether every entry stays below
-//     random::COUNT_LIMIT whatever the draws;
+//   count_update(time, dt, c, shared, rng): one update in place, on the
+//     state as FP32 counts c[0], c[1], ..., giving exactly what update()
+//     does (c is a float* or a strided_counts);
+//   count_fits(c): whether every entry stays below random::COUNT_LIMIT
+//     whatever the draws;
 //   count_prepare(shared_state&, dt) (host): fills shared.counts, whose
 //     member `ready(dt)` says whether the group can be stepped this way.
+// A large state may declare its own layout instead of count_fits:
+//   count_size: the entries of c, which need not be the state's;
+//   count_load(g, c): fills c from the state g[s] (doubles in device
+//     memory), and says whether it is counts that fit;
+//   count_store(g, c): brings g up to date from c and what g held at the
+//     last load or store.  It runs before a zero_every reset, which then
+//     acts on g (and must not touch entries that c holds).
 // A particle whose entries are not all counts, or that does not fit, is
 // stepped by update().
 template <class T, class = void>
 struct has_count_update : std::false_type {};
 template <class T>
-struct has_count_update<T, std::void_t<decltype(&T::count_update)>>
+struct has_count_update<T, std::void_t<decltype(&T::count_prepare)>>
   : std::true_type {};
+
+template <class T, class = void>
+struct has_count_layout : std::false_type {};
+template <class T>
+struct has_count_layout<T, std::void_t<decltype(T::count_size)>>
+  : std::true_type {};
+
+// Entries of c.
+template <typename T>
+constexpr int count_size_of() {
+  if constexpr (has_count_layout<T>::value) {
+    return T::count_size;
+  } else {
+    return T::n_state_max;
+  }
+}
+
+// One thread's counts in a block's shared memory, entry by entry (no bank
+// conflicts).  quad(first, i) is four integers in the place of the entries
+// from first + 4 i, read and written in one instruction.
+struct alignas(16) count_quad {
+  std::uint32_t v[4];
+};
+struct strided_counts {
+  float* base;
+  int stride;
+  int thread;
+  DUST2_HD float& operator[](int s) const {
+    return base[s * stride + thread];
+  }
+  DUST2_HD count_quad& quad(int first, int i) const {
+    return reinterpret_cast<count_quad*>(base + first * stride)
+      [i * stride + thread];
+  }
+};
 
 // The shared state as a kernel sees it: with the count tables of `dt`.
 template <typename T>

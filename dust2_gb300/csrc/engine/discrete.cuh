@@ -95,7 +95,7 @@ struct shared_smem {
            base += 32) {
         const int i = base + lane;
         const double t = time + static_cast<double>(i) * dt;
-        const bool hit = i < n_steps && fmod(t, z.period[e]) == 0;
+        const bool hit = i < n_steps && math::is_multiple(t, z.period[e]);
         mask |= static_cast<std::uint64_t>(__ballot_sync(0xffffffffu, hit))
           << base;
       }
@@ -128,17 +128,43 @@ __device__ __forceinline__ void store_state(const system_view<T>& v, int k,
   }
 }
 
+// Whether entry i of the zero_every table is due at step `step`.
+__device__ __forceinline__ bool zero_every_hit(
+    const zero_every_spec& z, const std::uint64_t* zero_steps, int step,
+    double time, int i) {
+  return (zero_steps != nullptr && step < ZERO_STEPS_CACHED) ?
+    ((zero_steps[i] >> step) & 1) != 0 :
+    math::is_multiple(time, z.period[i]);
+}
+
+__device__ __forceinline__ bool zero_every_due(
+    const zero_every_spec& z, const std::uint64_t* zero_steps, int step,
+    double time) {
+  bool due = false;
+  for (int i = 0; i < z.n; ++i) {
+    due = due || zero_every_hit(z, zero_steps, step, time, i);
+  }
+  return due;
+}
+
+// One particle's state in device memory.
+struct state_column {
+  double* p;
+  long stride;
+  __device__ __forceinline__ double& operator[](int s) const {
+    return p[s * stride];
+  }
+};
+
 // Reset the zero_every entries due at step `step` (time `time`): the
 // first ZERO_STEPS_CACHED steps read the block's precomputed masks.  The
 // state is doubles, or FP32 counts.
-template <typename T, typename R>
+template <typename T, typename C>
 __device__ __forceinline__ void apply_zero_every(
     const zero_every_spec& z, const std::uint64_t* zero_steps, int step,
-    double time, R* x) {
+    double time, C&& x) {
   for (int i = 0; i < z.n; ++i) {
-    const bool hit = (zero_steps != nullptr && step < ZERO_STEPS_CACHED) ?
-      ((zero_steps[i] >> step) & 1) != 0 : fmod(time, z.period[i]) == 0;
-    if (hit) {
+    if (zero_every_hit(z, zero_steps, step, time, i)) {
       if constexpr (T::n_state_max > 32) {
         // a large state lives in local memory: walk the mask's set bits
         // (an unrolled test of every entry made the compiler keep entries
@@ -225,6 +251,53 @@ __device__ __noinline__ void step_particle_update(
   store_state<T>(v, k, x);
 }
 
+// Pick a block size for a system: big states need more registers per
+// thread, so fewer threads per block keep occupancy sane.  Every kernel
+// over a system's particles runs with this block size.
+template <typename T>
+constexpr int default_tile_size() {
+  return T::n_state_max > 32 ? 128 : 256;
+}
+
+// Where a thread keeps its counts: registers, or for a state too large for
+// them the block's dynamic shared memory (in local memory SEIR's 96 entries
+// missed the L1 cache half the time).
+template <typename T>
+constexpr int count_smem_per_thread() {
+  return has_count_update<T>::value && T::n_state_max > 32 ?
+    static_cast<int>(count_size_of<T>() * sizeof(float)) : 0;
+}
+
+template <int N>
+struct register_counts {
+  mutable float x[N];
+  __device__ __forceinline__ float& operator[](int s) const {
+    return x[s];
+  }
+};
+
+template <typename T>
+__device__ __forceinline__ auto thread_counts() {
+  if constexpr (count_smem_per_thread<T>() > 0) {
+    extern __shared__ count_quad count_smem[];
+    return strided_counts{reinterpret_cast<float*>(count_smem),
+                          static_cast<int>(blockDim.x),
+                          static_cast<int>(threadIdx.x)};
+  } else {
+    return register_counts<T::n_state_max>{};
+  }
+}
+
+// Let `kernel` use that much dynamic shared memory at the largest block.
+template <typename T, typename K>
+void allow_count_smem(K kernel) {
+  if constexpr (count_smem_per_thread<T>() > 0) {
+    DUST2_CUDA(cudaFuncSetAttribute(
+      kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      count_smem_per_thread<T>() * default_tile_size<T>()));
+  }
+}
+
 // Advance particle k n_steps from its state in device memory and store
 // it again; then done(x, internal) runs on the new state.  Systems with
 // count_update step a particle whose state is counts in FP32
@@ -239,30 +312,45 @@ __device__ __forceinline__ void step_particle(
   typename T::internal_state internal{};
   double x[T::n_state_max];
   if constexpr (has_count_update<T>::value) {
-    float c[T::n_state_max];
+    const auto c = thread_counts<T>();
     bool ok = !v.deterministic && shared.counts.ready(dt);
-    if (ok) {
+    const state_column g{v.state + k, v.stride};
+    if constexpr (has_count_layout<T>::value) {
+      ok = ok && T::count_load(g, c);
+    } else if (ok) {
 #pragma unroll
       for (int s = 0; s < T::n_state_max; ++s) {
-        c[s] = 0;
+        float f = 0;
         if (s < v.n_state) {
-          ok &= random::filter::count_of(
-            v.state[static_cast<long>(s) * v.stride + k], &c[s]);
+          ok &= random::filter::count_of(g[s], &f);
         }
+        c[s] = f;
       }
       ok = ok && T::count_fits(c);
     }
     if (ok) {
       for (int i = 0; i < n_steps; ++i) {
         const double t = time + static_cast<double>(i) * dt;
-        apply_zero_every<T>(z, zero_steps, i, t, c);
+        if constexpr (has_count_layout<T>::value) {
+          if (i > 0 && zero_every_due(z, zero_steps, i, t)) {
+            T::count_store(g, c);
+          }
+          apply_zero_every<T>(z, zero_steps, i, t, g);
+        } else {
+          apply_zero_every<T>(z, zero_steps, i, t, c);
+        }
         T::count_update(t, dt, c, shared, rng);
       }
+      if constexpr (has_count_layout<T>::value) {
+        T::count_store(g, c);
+        load_state<T>(v, k, x);  // the entries that done() reads
+      } else {
 #pragma unroll
-      for (int s = 0; s < T::n_state_max; ++s) {
-        if (s < v.n_state) {
-          x[s] = random::filter::count_to_double(c[s]);
-          v.state[static_cast<long>(s) * v.stride + k] = x[s];
+        for (int s = 0; s < T::n_state_max; ++s) {
+          if (s < v.n_state) {
+            x[s] = random::filter::count_to_double(c[s]);
+            g[s] = x[s];
+          }
         }
       }
     } else {
@@ -270,10 +358,6 @@ __device__ __forceinline__ void step_particle(
       step_particle_update<T>(v, k, time, dt, n_steps, shared, z, zero_steps,
                               r);
       rng = r;
-      load_state<T>(v, k, x);
-    }
-    if constexpr (T::n_state_max > 32) {
-      // too large for registers: `done` reads what it needs from memory
       load_state<T>(v, k, x);
     }
   } else {
@@ -284,14 +368,6 @@ __device__ __forceinline__ void step_particle(
     store_state<T>(v, k, x);
   }
   done(x, internal);
-}
-
-// Pick a block size for a system: big states need more registers per
-// thread, so fewer threads per block keep occupancy sane.  Every kernel
-// over a system's particles runs with this block size.
-template <typename T>
-constexpr int default_tile_size() {
-  return T::n_state_max > 32 ? 128 : 256;
 }
 
 // The tile size for a set of groups: the system's block size, halved
@@ -464,6 +540,9 @@ public:
     if (n_state_ > T::n_state_max) {
       throw std::runtime_error("state larger than the system's n_state_max");
     }
+    if constexpr (!dust2gpu::is_continuous<T>()) {
+      allow_count_smem<T>(k_run<T>);
+    }
     DUST2_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     const int stride = layout_.stride;
     state_.resize(static_cast<std::size_t>(n_state_) * stride);
@@ -627,7 +706,9 @@ public:
   void launch_run(double t0, int n_steps) {
     if constexpr (has_update<T>::value && !dust2gpu::is_continuous<T>()) {
       if (n_steps > 0) {
-        k_run<T><<<n_run_tiles(), layout_.tile_size, 0, stream_>>>(
+        k_run<T><<<n_run_tiles(), layout_.tile_size,
+                   count_smem_per_thread<T>() * layout_.tile_size,
+                   stream_>>>(
           run_view(), t0, dt_, n_steps);
         DUST2_CUDA(cudaGetLastError());
       }

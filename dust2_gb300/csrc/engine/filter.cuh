@@ -141,6 +141,32 @@ DUST2_PARTICLE_KERNEL(T) k_initial_flagged(system_view<T> v, const int* flag,
   capture_error(v.errors, v.any_error, k, rng);
 }
 
+// Add a warp's log weights to its group's reductions: "any weight
+// non-zero" and the maximum, both by atomics and on the integer bits.
+// NaN != 0 counts as data (filter.hpp:71-72); NaN is -Inf for the max.
+// Each warp reduces for itself: when the block did, its warps waited for
+// the slowest (2.0 of the SIR kernel's 8.3 cycles per issue).
+__device__ __forceinline__ void reduce_weight(const filter_view& f, int group,
+                                              bool valid, double logw) {
+  constexpr unsigned all = 0xffffffffu;
+  const std::uint64_t bits = math::bits_of(logw);
+  const unsigned nz = __ballot_sync(all, valid && (bits << 1) != 0);
+  const bool number = (bits << 1) <= 0xffe0000000000000ull;
+  const unsigned long long key =
+    ordered_key(valid && number ? logw : -INFINITY);
+  const unsigned hi = static_cast<unsigned>(key >> 32);
+  const unsigned top = __reduce_max_sync(all, hi);
+  const unsigned low = __reduce_max_sync(
+    all, hi == top ? static_cast<unsigned>(key) : 0u);
+  if ((threadIdx.x & 31) == 0) {
+    if (nz != 0) {
+      atomicOr(f.gnz + group, 1);
+    }
+    atomicMax(f.gkey + group,
+              (static_cast<unsigned long long>(top) << 32) | low);
+  }
+}
+
 // The per-tile work of k_step_compare, shared with the likelihood
 // server: advance each particle of tile `tl` n_steps from `time`, compare
 // it with `d` (this tile's data row), store its log weight, and reduce the
@@ -148,7 +174,7 @@ DUST2_PARTICLE_KERNEL(T) k_initial_flagged(system_view<T> v, const int* flag,
 template <typename T>
 __device__ __forceinline__ void step_compare_tile(
     const system_view<T>& v, const filter_view& f, const tile& tl,
-    shared_smem<T>& sm, double* red, double time, double dt, int n_steps,
+    shared_smem<T>& sm, double time, double dt, int n_steps,
     double time_compare, const typename T::data_type* d) {
   sm.load(v, tl.group);
   sm.load_zero_steps(v, tl.group, time, dt, n_steps);
@@ -168,16 +194,7 @@ __device__ __forceinline__ void step_compare_tile(
     capture_error(v.errors, v.any_error, k, rng);
     f.w[k] = logw;
   }
-  // NaN != 0 counts as data (filter.hpp:71-72); NaN is -Inf for the max.
-  const int nz = __syncthreads_or(valid && logw != 0);
-  const double mx = block_max(valid && !(logw != logw) ? logw : -INFINITY,
-                              red);
-  if (threadIdx.x == 0) {
-    if (nz) {
-      atomicOr(f.gnz + tl.group, 1);
-    }
-    atomicMax(f.gkey + tl.group, ordered_key(mx));
-  }
+  reduce_weight(f, tl.group, valid, logw);
 }
 
 // k_step_compare for mixed-time systems (filter.hpp:59-60 over
@@ -194,7 +211,6 @@ DUST2_PARTICLE_KERNEL(T) k_step_compare_mixed(
     const typename T::data_type* data, int n_groups_data) {
   constexpr int NV = n_var_max<T>();
   __shared__ shared_smem<T> sm;
-  __shared__ double red[33];
   const tile tl = v.tiles[blockIdx.x];
   if (!f.active[tl.group]) {
     return;
@@ -234,15 +250,7 @@ DUST2_PARTICLE_KERNEL(T) k_step_compare_mixed(
     capture_error(v.errors, v.any_error, k, rng);
     f.w[k] = logw;
   }
-  const int nz = __syncthreads_or(valid && logw != 0);
-  const double mx = block_max(valid && !(logw != logw) ? logw : -INFINITY,
-                              red);
-  if (threadIdx.x == 0) {
-    if (nz) {
-      atomicOr(f.gnz + tl.group, 1);
-    }
-    atomicMax(f.gkey + tl.group, ordered_key(mx));
-  }
+  reduce_weight(f, tl.group, valid, logw);
 }
 
 template <typename T>
@@ -252,12 +260,11 @@ DUST2_PARTICLE_KERNEL(T) k_step_compare(system_view<T> v, filter_view f,
                                const typename T::data_type* data,
                                int n_groups_data) {
   __shared__ shared_smem<T> sm;
-  __shared__ double red[33];
   const tile tl = v.tiles[blockIdx.x];
   if (!f.active[tl.group]) {
     return;
   }
-  step_compare_tile<T>(v, f, tl, sm, red, time, dt, n_steps, time_compare,
+  step_compare_tile<T>(v, f, tl, sm, time, dt, n_steps, time_compare,
                        data + (n_groups_data == 1 ? 0 : tl.group));
 }
 
@@ -272,9 +279,9 @@ DUST2_PARTICLE_KERNEL(T) k_step_compare_queue(
     double time_compare, const typename T::data_type* data,
     int n_groups_data, int n_tiles, int* next_tile) {
   __shared__ shared_smem<T> sm;
-  __shared__ double red[33];
   __shared__ int taken;
   for (;;) {
+    __syncthreads();  // every warp is done with the last tile's `sm`
     if (threadIdx.x == 0) {
       taken = atomicAdd(next_tile, 1);
     }
@@ -288,8 +295,7 @@ DUST2_PARTICLE_KERNEL(T) k_step_compare_queue(
     if (!f.active[tl.group]) {
       continue;
     }
-    step_compare_tile<T>(v, f, tl, sm, red, time, dt, n_steps,
-                         time_compare,
+    step_compare_tile<T>(v, f, tl, sm, time, dt, n_steps, time_compare,
                          data + (n_groups_data == 1 ? 0 : tl.group));
   }
 }
@@ -438,6 +444,8 @@ public:
     sys_->sync();
     set_fused_tail(true);
     if constexpr (!is_continuous<T>()) {
+      allow_count_smem<T>(k_step_compare<T>);
+      allow_count_smem<T>(k_step_compare_queue<T>);
       queue_.resize(std::max<std::size_t>(1, schedule_.size()));
       set_shape(default_shape());
     }
@@ -926,7 +934,8 @@ public:
   int persistent_grid(int block, int n_tiles) const {
     int per_sm = 0;
     DUST2_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &per_sm, k_step_compare_queue<T>, block, 0));
+      &per_sm, k_step_compare_queue<T>, block,
+      count_smem_per_thread<T>() * block));
     return std::max(1, std::min(n_tiles, std::max(1, per_sm) * n_sms()));
   }
 
@@ -954,12 +963,13 @@ public:
                          std::size_t i, int* next_tile) {
     auto& S = *sys_;
     const auto* d = data_.data() + i * n_groups_data_;
+    const int smem = count_smem_per_thread<T>() * sh.block;
     if (sh.persistent) {
-      k_step_compare_queue<T><<<grid, sh.block, 0, s>>>(
+      k_step_compare_queue<T><<<grid, sh.block, smem, s>>>(
         v, f, st.t0, S.dt(), st.n_steps, st.t_compare, d, n_groups_data_,
         n_tiles, next_tile);
     } else {
-      k_step_compare<T><<<n_tiles, sh.block, 0, s>>>(
+      k_step_compare<T><<<n_tiles, sh.block, smem, s>>>(
         v, f, st.t0, S.dt(), st.n_steps, st.t_compare, d, n_groups_data_);
     }
   }
@@ -1071,8 +1081,9 @@ public:
     }
     steps = std::min(steps, 400);
     if (steps > 0) {
-      k_run<T><<<run_tiles, L.tile_size, 0, s>>>(v, time_start_, S.dt(),
-                                                 steps);
+      k_run<T><<<run_tiles, L.tile_size,
+                 count_smem_per_thread<T>() * L.tile_size, s>>>(
+        v, time_start_, S.dt(), steps);
     }
     DUST2_CUDA(cudaGetLastError());
     const double t0 = time_start_ + steps * S.dt();

@@ -133,7 +133,6 @@ DUST2_PARTICLE_KERNEL(T) k_served_step_compare(system_view<T> v,
                                       const typename T::data_type* data,
                                       int* slot_error) {
   __shared__ shared_smem<T> sm;
-  __shared__ double red[33];
   const tile tl = v.tiles[blockIdx.x];
   const int g = tl.group;
   if (!f.active[g]) {
@@ -144,7 +143,7 @@ DUST2_PARTICLE_KERNEL(T) k_served_step_compare(system_view<T> v,
   const obs_step st = sched[sl.sched_offset + o];
   system_view<T> vs = v;
   vs.any_error = slot_error + g;
-  step_compare_tile<T>(vs, f, tl, sm, red, st.t0, sl.dt, st.n_steps,
+  step_compare_tile<T>(vs, f, tl, sm, st.t0, sl.dt, st.n_steps,
                        st.t_compare, data + sl.data_offset + o);
 }
 
@@ -320,6 +319,7 @@ public:
     }
     max_tiles_ = cap_particles_ / ALIGN + n_slots_;
 
+    allow_count_smem<T>(k_served_step_compare<T>);
     DUST2_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     const std::size_t P = cap_particles_;
     const std::size_t S = n_slots_;
@@ -989,7 +989,7 @@ private:
     if (timed) {
       DUST2_CUDA(cudaEventRecord(r.step0, s));
     }
-    k_served_step_compare<T><<<NT, TS, 0, s>>>(
+    k_served_step_compare<T><<<NT, TS, count_smem_per_thread<T>() * TS, s>>>(
       sview(cur()), f, slots_dev_.data(), obs_dev_.data(), sched_.data(),
       data_.data(), slot_error_.data());
     if (timed) {

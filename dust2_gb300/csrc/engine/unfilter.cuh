@@ -282,7 +282,7 @@ DUST2_PARTICLE_KERNEL(T) k_unfilter_adjoint(
           adj[a] = adj_next[a];
         }
         for (int e = 0; e < zero.n; ++e) {
-          if (fmod(time_b, zero.period[e]) == 0) {
+          if (math::is_multiple(time_b, zero.period[e])) {
             for (int s = 0; s < ns; ++s) {
               if (zero.has(e, s)) {
                 adj[s] = 0;

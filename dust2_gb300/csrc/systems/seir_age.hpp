@@ -23,15 +23,12 @@ struct seir_age {
   // it has written: it is correct in place, so a particle keeps one
   // state array.
   static constexpr bool update_in_place = true;
-  // The 96 doubles stay in a per-thread array (local memory, cached),
-  // with 4 blocks of 128 threads per SM (128 registers).  Measured on
-  // the batched SEIR filter (particle-steps/s): this 149.5M; 3 blocks
-  // 144.3M; 5 blocks 147.3M.  Earlier builds: two arrays with copies
-  // (before in-place updates) 116.0M against 118.2M in place; the state
-  // in rows of shared memory instead (2 blocks of 99 KB per SM) 107.7M --
-  // occupancy hides the FP64 pipe's latency better than shared memory
-  // saves local-memory traffic.
-  static constexpr int min_blocks_per_sm = 4;
+  // 5 blocks of 128 threads per SM: 96 registers, and 160 KB of shared
+  // memory for the counts.  32 groups x 8192 particles, 60 observations:
+  // 4 blocks 77.1 ms, 5 72.5, 6 92.5 (the L1 cache that is left no longer
+  // holds what 80 registers spill).  All 96 entries as FP32 in local
+  // memory (L1 hit rate 49%) 84.0 ms, in shared memory 88.5.
+  static constexpr int min_blocks_per_sm = 5;
   using real_type = double;
   using rng_state_type = random::rng_state;
   static constexpr int n_age = 16;
@@ -45,8 +42,7 @@ struct seir_age {
   // many FP64 ones (76 cycles).
   struct count_table {
     std::uint64_t key_dt;
-    random::count_prob e_i;
-    random::count_prob i_r;
+    random::count_prob after[2];  // E to I, I to R
     bool ok;
     int scale[n_age];
     alignas(16) std::uint32_t k[n_age][n_age];
@@ -238,9 +234,9 @@ struct seir_age {
   static void count_prepare(shared_state& s, real_type dt) {
     count_table& c = s.counts;
     c.key_dt = math::bits_of(dt);
-    c.e_i = random::make_count_prob(1 - math::exp(-s.sigma * dt));
-    c.i_r = random::make_count_prob(1 - math::exp(-s.gamma * dt));
-    c.ok = c.e_i.ok && c.i_r.ok;
+    c.after[0] = random::make_count_prob(1 - math::exp(-s.sigma * dt));
+    c.after[1] = random::make_count_prob(1 - math::exp(-s.gamma * dt));
+    c.ok = c.after[0].ok && c.after[1].ok;
     for (int a = 0; a < n_age && c.ok; ++a) {
       double row[n_age];
       double top = 0;
@@ -260,79 +256,131 @@ struct seir_age {
     }
   }
 
+  // Stepped are S, E and I, and the I of the step's start as integers: 256
+  // bytes a particle, in shared memory.  What has flowed into R and the
+  // two case counts since they were last stored follows from what S, E and
+  // I were then.
+  static constexpr int count_size = 4 * n_age;
+
   // Within an age nothing exceeds the sum of its entries.
-  DUST2_HD static bool count_fits(const float* c) {
-    float top = 0;
+  template <typename G, typename C>
+  DUST2_HD static bool count_load(const G& g, C&& c) {
+    bool ok = true;
+#pragma unroll
     for (int a = 0; a < n_age; ++a) {
       float sum = 0;
       for (int j = 0; j < 6; ++j) {
-        sum += c[j * n_age + a];
+        float f = 0;
+        ok &= random::filter::count_of(g[j * n_age + a], &f);
+        sum += f;
+        if (j < 3) {
+          c[j * n_age + a] = f;
+        }
       }
-      top = std::fmax(top, sum);
+      ok &= sum < random::COUNT_LIMIT;
     }
-    return top < random::COUNT_LIMIT;
+    return ok;
+  }
+
+  template <typename G, typename C>
+  DUST2_HD static void count_store(G&& g, C&& c) {
+#pragma unroll
+    for (int a = 0; a < n_age; ++a) {
+      float was[6];
+      for (int j = 0; j < 6; ++j) {
+        random::filter::count_of(g[j * n_age + a], &was[j]);
+      }
+      const float S = c[a];
+      const float E = c[n_age + a];
+      const float I = c[2 * n_age + a];
+      const float n_EI = (was[0] + was[1]) - (S + E);
+      const float n_IR = (was[2] + n_EI) - I;
+      g[a] = random::filter::count_to_double(S);
+      g[n_age + a] = random::filter::count_to_double(E);
+      g[2 * n_age + a] = random::filter::count_to_double(I);
+      g[3 * n_age + a] = random::filter::count_to_double(was[3] + n_IR);
+      g[4 * n_age + a] = random::filter::count_to_double(was[4] + n_EI);
+      g[5 * n_age + a] = random::filter::count_to_double(was[5] + n_EI);
+    }
   }
 
   // 1 - exp(-lambda_a dt) as update() forms it.
+  template <typename C>
   DUST2_SAMPLER static real_type p_SE_fp64(const shared_state& shared,
-                                           const float* I, int a,
+                                           const C& c, int a,
                                            real_type dt) {
     real_type acc = 0;
     for (int b = 0; b < n_age; ++b) {
+      const std::uint32_t I = c.quad(3 * n_age, b / 4).v[b % 4];
       const real_type x =
-        random::filter::count_to_double(I[b]) * shared.inv_N[b];
+        random::filter::count_to_double(static_cast<float>(I)) *
+        shared.inv_N[b];
       acc = std::fma(shared.contact[a][b], x, acc);
     }
     const real_type lambda = shared.beta * acc;
     return 1 - math::exp(-lambda * dt);
   }
 
-  DUST2_HD static void count_update(real_type time, real_type dt, float* c,
+  template <typename C>
+  DUST2_HD static void count_update(real_type time, real_type dt, C&& c,
                                     const shared_state& shared,
                                     rng_state_type& rng_state) {
     const count_table& tab = shared.counts;
-    float I_start[n_age];  // for the FP64 probability, when it is needed
-    std::uint32_t I_int[n_age];
     std::uint32_t I_sum = 0;
 #pragma unroll
-    for (int b = 0; b < n_age; ++b) {
-      I_start[b] = c[2 * n_age + b];
-      I_int[b] = static_cast<std::uint32_t>(I_start[b]);
-      I_sum += I_int[b];
+    for (int q = 0; q < n_age / 4; ++q) {
+      count_quad I;
+      for (int j = 0; j < 4; ++j) {
+        I.v[j] = static_cast<std::uint32_t>(c[2 * n_age + 4 * q + j]);
+        I_sum += I.v[j];
+      }
+      c.quad(3 * n_age, q) = I;
     }
     const float half_sum = 0.501f * static_cast<float>(I_sum);
 #pragma unroll 1
     for (int a = 0; a < n_age; ++a) {
       std::uint64_t acc = 0;
 #pragma unroll
-      for (int b = 0; b < n_age; ++b) {
-        acc += static_cast<std::uint64_t>(tab.k[a][b]) * I_int[b];
+      for (int q = 0; q < n_age / 4; ++q) {
+        const count_quad I = c.quad(3 * n_age, q);
+        const count_quad k =
+          reinterpret_cast<const count_quad*>(tab.k[a])[q];
+        for (int j = 0; j < 4; ++j) {
+          acc += static_cast<std::uint64_t>(k.v[j]) * I.v[j];
+        }
       }
       const float S = c[a];
       const float E = c[n_age + a];
       const float I = c[2 * n_age + a];
-      float n_SE = 0;
-      if (I_sum != 0) {
-        // a hazard of 1/2 or more is passed on as such
-        const int scale = tab.scale[a];
-        const std::uint64_t x62 =
-          (acc >> (scale - 1)) != 0 ? ~0ull : acc << (62 - scale);
-        const float units =
-          std::fmaf(static_cast<float>(static_cast<std::uint32_t>(acc >> 32)),
-                    0x1p32f,
-                    static_cast<float>(static_cast<std::uint32_t>(acc)));
-        n_SE = random::binomial_hazard(
-          rng_state, S, x62, half_sum * random::filter::rcp32(units),
-          [&] { return p_SE_fp64(shared, I_start, a, dt); });
+      // a hazard of 1/2 or more is passed on as such
+      const int scale = tab.scale[a];
+      const std::uint64_t x62 =
+        (acc >> (scale - 1)) != 0 ? ~0ull : acc << (62 - scale);
+      const float units =
+        std::fmaf(static_cast<float>(static_cast<std::uint32_t>(acc >> 32)),
+                  0x1p32f,
+                  static_cast<float>(static_cast<std::uint32_t>(acc)));
+      random::draw_prob d = random::hazard_draw(
+        x62, half_sum * random::filter::rcp32(units));
+      d.zero = I_sum == 0;
+      float n = S;
+      float n_SE = 0, n_EI = 0, n_IR = 0;
+#pragma unroll 1
+      for (int j = 0; j < 3; ++j) {
+        const float k = random::draw_count(rng_state, n, d, [&] {
+          return j == 0 ? p_SE_fp64(shared, c, a, dt) : tab.after[j - 1].p;
+        });
+        if (j < 2) {
+          d = tab.after[j].d;
+        }
+        n = j == 0 ? E : I;
+        n_SE = j == 0 ? k : n_SE;
+        n_EI = j == 1 ? k : n_EI;
+        n_IR = k;
       }
-      const float n_EI = random::binomial_count(rng_state, E, tab.e_i);
-      const float n_IR = random::binomial_count(rng_state, I, tab.i_r);
       c[a] = S - n_SE;
       c[n_age + a] = E + n_SE - n_EI;
       c[2 * n_age + a] = I + n_EI - n_IR;
-      c[3 * n_age + a] = c[3 * n_age + a] + n_IR;
-      c[4 * n_age + a] = c[4 * n_age + a] + n_EI;
-      c[5 * n_age + a] = c[5 * n_age + a] + n_EI;
     }
   }
 

@@ -28,27 +28,41 @@ struct sir_counts {
     return ok && key_dt == math::bits_of(dt);
   }
 
-  // I < 2^24 and rate < 1: a hazard of 2 or more would wrap, so it is
+  // I < 2^24 and rate < 1: a hazard of 4 or more would wrap, so it is
   // bounded in FP32 first (any hazard of 1/2 or more takes the FP64
   // probability).
   DUST2_HD void draw(random::rng_state& rng, float S, float I, double N,
                      double beta, double dt, float* n_SI,
                      float* n_IR) const {
-    *n_SI = 0;
-    if (I > 0.0f) {
-      const std::uint32_t rate_hi = static_cast<std::uint32_t>(rate62 >> 38);
-      const std::uint64_t x62 =
-        I * (static_cast<float>(rate_hi) + 1.0f) < 0x1p24f ?
-        static_cast<std::uint32_t>(I) * rate62 : ~0ull;
-      *n_SI = random::binomial_hazard(rng, S, x62, 0.0f, [&] {
-        return 1 - math::exp(-beta * filter_to_double(I) / N * dt);
+    const std::uint32_t rate_hi = static_cast<std::uint32_t>(rate62 >> 38);
+    const std::uint64_t x62 =
+      I * (static_cast<float>(rate_hi) + 1.0f) < 0x1p24f ?
+      static_cast<std::uint32_t>(I) * rate62 : ~0ull;
+    random::draw_prob d = random::hazard_draw(x62, 0.0f);
+    d.zero = I == 0.0f;
+    float n = S;
+    float first = 0;
+    // the body holds a sampler: one copy for both draws
+#pragma unroll 1
+    for (int j = 0;; ++j) {
+      const float k = random::draw_count(rng, n, d, [&] {
+        return j == 0 ? p_SI(I, N, beta, dt) : recover.p;
       });
+      if (j == 1) {
+        *n_SI = first;
+        *n_IR = k;
+        return;
+      }
+      first = k;
+      n = I;
+      d = recover.d;
     }
-    *n_IR = random::binomial_count(rng, I, recover);
   }
 
-  DUST2_HD static double filter_to_double(float x) {
-    return random::filter::count_to_double(x);
+  // As update() forms it.
+  DUST2_SAMPLER static double p_SI(float I, double N, double beta,
+                                   double dt) {
+    return 1 - math::exp(-beta * random::filter::count_to_double(I) / N * dt);
   }
 };
 

@@ -30,14 +30,23 @@ static unsigned long long steps, wrong, unfit;
 template <typename T>
 void run(const typename T::shared_state& shared, const double* start,
          int n_state, double dt, int n_steps, random::rng_state rng) {
-  float c[T::n_state_max] = {};
-  double x[T::n_state_max] = {}, y[T::n_state_max];
-  bool ok = shared.counts.ready(dt);
+  constexpr int size = count_size_of<T>();
+  alignas(16) float cells[size] = {};
+  const strided_counts c{cells, 1, 0};
+  double x[T::n_state_max] = {}, y[T::n_state_max], g[T::n_state_max];
   for (int s = 0; s < n_state; ++s) {
-    x[s] = start[s];
-    ok = ok && random::filter::count_of(x[s], &c[s]);
+    g[s] = x[s] = start[s];
   }
-  if (!ok || !T::count_fits(c)) {
+  bool ok = shared.counts.ready(dt);
+  if constexpr (has_count_layout<T>::value) {
+    ok = ok && T::count_load(g, c);
+  } else {
+    for (int s = 0; s < n_state; ++s) {
+      ok = ok && random::filter::count_of(x[s], &c[s]);
+    }
+    ok = ok && T::count_fits(c);
+  }
+  if (!ok) {
     ++unfit;
     return;
   }
@@ -46,11 +55,20 @@ void run(const typename T::shared_state& shared, const double* start,
   for (int i = 0; i < n_steps; ++i) {
     T::count_update(i * dt, dt, c, shared, a);
     T::update(i * dt, dt, x, shared, internal, b, y);
+    if constexpr (has_count_layout<T>::value) {
+      if (i % 3 != 1) {  // stored after every step or after two
+        T::count_store(g, c);
+      }
+    } else {
+      for (int s = 0; s < n_state; ++s) {
+        g[s] = random::filter::count_to_double(c[s]);
+      }
+    }
     bool same = true;
     for (int s = 0; s < n_state; ++s) {
       x[s] = y[s];
-      same = same && math::bits_of(random::filter::count_to_double(c[s])) ==
-        math::bits_of(x[s]);
+      same = same && (i % 3 == 1 ||
+                      math::bits_of(g[s]) == math::bits_of(x[s]));
     }
     for (int w = 0; w < 4; ++w) {
       same = same && a.state[w] == b.state[w];
