@@ -569,6 +569,46 @@ DUST2_MATH_CORE double rcp(double y) {
   return std::fma(r, e, r);
 }
 
+// Exact division by a value that is used many times: a / b, correctly
+// rounded, in 4 FP64 instructions instead of an IEEE division's sequence.
+// With hi = RN(1/b) and lo = 1/b - hi, q = fma(a, hi, RN(a lo)) is within
+// an ulp of a / b, and with hi correctly rounded fma(fma(-q, b, a), hi, q)
+// is then RN(a / b) (Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34 (1990), theorem
+// 2), as long as nothing over- or underflows; other arguments divide.
+struct divisor {
+  double b;
+  double hi;
+  double lo;  // NaN: always divide
+
+  static divisor of(double b) {
+    divisor d{b, 1.0 / b, quiet_nan()};
+    const double m = std::fabs(b);
+    if (m > 0x1p-300 && m < 0x1p300) {
+      d.lo = std::fma(-d.hi, b, 1.0) / b;
+    }
+    return d;
+  }
+};
+
+DUST2_HD double divide_fma(double a, const divisor& d) {
+  const int e = static_cast<int>((bits_of(a) >> 52) & 0x7ff);
+  if (e < 1023 - 400 || e > 1023 + 400 ||
+      (bits_of(d.lo) << 1) > 0xffe0000000000000ull) {
+    return a / d.b;
+  }
+  const double q = std::fma(a, d.hi, a * d.lo);
+  return std::fma(std::fma(-q, d.b, a), d.hi, q);
+}
+
+DUST2_HD double divide(double a, const divisor& d) {
+#if defined(__CUDA_ARCH__)
+  return divide_fma(a, d);
+#else
+  return a / d.b;
+#endif
+}
+
 // 1/x for integer x in [1, 128] (correctly rounded, from a table).
 DUST2_HD double recip_int(int x) {
   return DUST2_TAB(recip_int, x);

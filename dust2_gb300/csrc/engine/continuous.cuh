@@ -81,6 +81,10 @@ __device__ __forceinline__ void load_ode(const ode_view& o, int k, int n_var,
   st.n_steps_accepted = o.n_steps_accepted[k];
   st.n_steps_rejected = o.n_steps_rejected[k];
   st.err = 0;
+  st.pending = false;
+  st.c4_set = 0;
+  st.has_log_error = false;
+  st.log_error = 0;
 }
 
 template <int NV>
@@ -106,6 +110,41 @@ __device__ __forceinline__ void store_ode(const ode_view& o, int k, int n_var,
   o.n_steps[k] = st.n_steps;
   o.n_steps_accepted[k] = st.n_steps_accepted;
   o.n_steps_rejected[k] = st.n_steps_rejected;
+}
+
+// Move every particle's solver record from src to dst, as k_reorder moves
+// its state; the rows are shared out over the grid's second dimension.
+template <int NV>
+__global__ void k_reorder_record(ode_view src, ode_view dst,
+                                 const tile* __restrict__ tiles,
+                                 const int* __restrict__ group_offset,
+                                 const int* __restrict__ index,
+                                 const int* __restrict__ group_mode) {
+  const tile tl = tiles[blockIdx.x];
+  if (static_cast<int>(threadIdx.x) >= tl.count) {
+    return;
+  }
+  const int k = tl.start + threadIdx.x;
+  const bool move = index != nullptr &&
+    (group_mode == nullptr || group_mode[tl.group] != 0);
+  const int from = move ? group_offset[tl.group] + index[k] : k;
+  const long S = src.stride;
+  for (int r = blockIdx.y; r < NV; r += gridDim.y) {
+    dst.dydt[r * S + k] = src.dydt[r * S + from];
+  }
+  for (int r = blockIdx.y; r < 5 * NV; r += gridDim.y) {
+    dst.c[r * S + k] = src.c[r * S + from];
+  }
+  if (blockIdx.y == 0) {
+    dst.t0[k] = src.t0[from];
+    dst.t1[k] = src.t1[from];
+    dst.h[k] = src.h[from];
+    dst.step_size[k] = src.step_size[from];
+    dst.error[k] = src.error[from];
+    dst.n_steps[k] = src.n_steps[from];
+    dst.n_steps_accepted[k] = src.n_steps_accepted[from];
+    dst.n_steps_rejected[k] = src.n_steps_rejected[from];
+  }
 }
 
 template <typename T>
@@ -239,6 +278,7 @@ __global__ void k_ode_run(system_view<T> v, ode_view o,
   }
   refresh_output<T>(t, y, shared, internal);
   store_state<T>(v, k, y);
+  sol.settle(st, s);
   store_ode<NV>(o, k, n_var, st);
   if (st.err != 0 || update_err != 0) {
     random::rng_state r{};
@@ -314,6 +354,7 @@ public:
     }
     requires_init_dev_.resize(base_.n_groups());
     other_.resize((6 * NV + 8) * S);
+    spread_tiles();
   }
 
   const char* name() const override {
@@ -415,14 +456,13 @@ public:
   void launch_unfilter(const double* times_dev, int n_times,
                        const int* active, const D* data, int n_groups_data,
                        double* ll, K kernel, const S& save) {
-    const auto& L = base_.layout();
     auto s = base_.stream();
     DUST2_CUDA(cudaMemcpyAsync(requires_init_dev_.data(),
                                requires_initialise_.data(),
                                requires_initialise_.size() * sizeof(int),
                                cudaMemcpyHostToDevice, s));
-    kernel<<<base_.n_run_tiles(), L.tile_size, 0, s>>>(
-      base_.run_view(), view_ode(), control_dev(), base_.time(), dt_,
+    kernel<<<n_ode_tiles_, ode_block_, 0, s>>>(
+      ode_run_view(), view_ode(), control_dev(), base_.time(), dt_,
       times_dev, n_times, requires_init_dev_.data(), active, data,
       n_groups_data, ll, save);
     DUST2_CUDA(cudaGetLastError());
@@ -456,7 +496,11 @@ public:
         DUST2_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
       }
     }
-    const int n_chunks = std::min(n_times, n_sim_chunks);
+    // (a small output is not worth a second launch)
+    const long n_chunks_worth = static_cast<long>(
+      per_time * n_times * sizeof(double) / (1 << 20)) + 1;
+    const int n_chunks = static_cast<int>(std::min<long>(
+      std::min(n_times, n_sim_chunks), n_chunks_worth));
     std::vector<int> first(n_chunks + 1);
     for (int c = 0; c <= n_chunks; ++c) {
       first[c] = static_cast<int>(static_cast<long>(n_times) * c / n_chunks);
@@ -632,41 +676,73 @@ public:
                     base_.layout().stride};
   }
 
-  // Enqueue the reordering of every particle's solver record on stream s
-  // (continuous/system.hpp:199-203, ode_internals moved with the state);
-  // arguments as k_reorder's.
-  void enqueue_reorder_record(const tile* tiles, int n_tiles, int tile_size,
+  // The solver records' second buffer, laid out in `other_`.
+  ode_view view_ode_other() {
+    const std::size_t S = base_.layout().stride;
+    double* p = other_.data();
+    int* n = reinterpret_cast<int*>(p + (6 * NV + 5) * S);
+    return ode_view{p, p + NV * S, p + 6 * NV * S, p + (6 * NV + 1) * S,
+                    p + (6 * NV + 2) * S, p + (6 * NV + 3) * S,
+                    p + (6 * NV + 4) * S, n, n + S, n + 2 * S,
+                    base_.layout().stride};
+  }
+
+  // Enqueue the reordering of every particle's solver record from src to
+  // dst on stream s (continuous/system.hpp:199-203, ode_internals moved
+  // with the state); arguments as k_reorder's, index null for a copy.
+  void enqueue_reorder_record(const ode_view& src, const ode_view& dst,
+                              const tile* tiles, int n_tiles, int tile_size,
                               const int* group_offset, const int* index,
                               const int* group_mode, cudaStream_t s) {
-    const int S = base_.layout().stride;
-    auto move = [&](double* a, int n_rows) {
-      k_reorder<<<n_tiles, tile_size, 0, s>>>(a, other_.data(), S, n_rows,
-                                              tiles, group_offset, index,
-                                              group_mode);
-      DUST2_CUDA(cudaMemcpyAsync(a, other_.data(),
-                                 static_cast<std::size_t>(n_rows) * S *
-                                 sizeof(double),
-                                 cudaMemcpyDeviceToDevice, s));
-    };
-    move(dydt_.data(), NV);
-    move(c_.data(), 5 * NV);
-    move(t0_.data(), 1);
-    move(t1_.data(), 1);
-    move(h_.data(), 1);
-    move(step_size_.data(), 1);
-    move(error_.data(), 1);
-    int* tmp = reinterpret_cast<int*>(other_.data());
-    for (int* a : {n_steps_.data(), n_acc_.data(), n_rej_.data()}) {
-      k_reorder_int<<<n_tiles, tile_size, 0, s>>>(a, tmp, S, tiles,
-                                                  group_offset, index,
-                                                  group_mode);
-      DUST2_CUDA(cudaMemcpyAsync(a, tmp, static_cast<std::size_t>(S) *
-                                 sizeof(int), cudaMemcpyDeviceToDevice, s));
-    }
+    k_reorder_record<NV><<<dim3(n_tiles, 16), tile_size, 0, s>>>(
+      src, dst, tiles, group_offset, index, group_mode);
     DUST2_CUDA(cudaGetLastError());
   }
 
 private:
+  // Tiles of the integrating kernels.  A problem with fewer warps of
+  // particles than the device has SM partitions (4 per SM) is cut into
+  // one-warp tiles of fewer particles: an FP64 instruction holds a
+  // partition as long for one lane as for 32, and particles that share a
+  // warp wait for each other's rejected and extra steps.
+  void spread_tiles() {
+    const auto& L = base_.layout();
+    ode_block_ = L.tile_size;
+    n_ode_tiles_ = base_.n_run_tiles();
+    int dev = 0, sms = 0;
+    DUST2_CUDA(cudaGetDevice(&dev));
+    DUST2_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount,
+                                      dev));
+    const int per = (L.n_total + 4 * sms - 1) / (4 * sms);
+    if (per >= 32) {
+      return;
+    }
+    std::vector<tile> tiles;
+    if (L.use_packed) {
+      for (int k = 0; k < L.n_total; k += per) {
+        const int count = std::min(per, L.n_total - k);
+        const int g = L.particle_group[k];
+        const bool one = L.particle_group[k + count - 1] == g;
+        tiles.push_back(tile{one ? g : -1, k, count, 0});
+      }
+    } else {
+      tiles = warp_tiles(L, per);
+    }
+    ode_tiles_.resize(tiles.size());
+    DUST2_CUDA(cudaMemcpy(ode_tiles_.data(), tiles.data(),
+                          tiles.size() * sizeof(tile),
+                          cudaMemcpyHostToDevice));
+    n_ode_tiles_ = static_cast<int>(tiles.size());
+    ode_block_ = 32;
+  }
+
+  system_view<T> ode_run_view() {
+    system_view<T> v = base_.run_view();
+    if (ode_tiles_.size() > 0) {
+      v.tiles = ode_tiles_.data();
+    }
+    return v;
+  }
 
   void launch_run(const double* times, int n_times, double* out_dev,
                   const int* index_dev, int n_out) {
@@ -682,8 +758,8 @@ private:
                                requires_initialise_.data(),
                                requires_initialise_.size() * sizeof(int),
                                cudaMemcpyHostToDevice, s));
-    k_ode_run<T><<<base_.n_run_tiles(), L.tile_size, 0, s>>>(
-      base_.run_view(), view_ode(), control_dev(), base_.time(), dt_,
+    k_ode_run<T><<<n_ode_tiles_, ode_block_, 0, s>>>(
+      ode_run_view(), view_ode(), control_dev(), base_.time(), dt_,
       times_dev_.data(), n_times, requires_init_dev_.data(), L.n_total,
       out_dev, index_dev, n_out);
     DUST2_CUDA(cudaGetLastError());
@@ -733,6 +809,9 @@ private:
   device_array<int> requires_init_dev_;
   device_array<double> times_dev_;
   device_array<double> other_;
+  device_array<tile> ode_tiles_;  // when spread over the device
+  int n_ode_tiles_ = 0;
+  int ode_block_ = 0;
   // simulate(): output buffer and the stream its chunks are copied on
   static constexpr int n_sim_chunks = 8;
   device_array<double> sim_buf_;

@@ -18,8 +18,9 @@
 // cut where the rounding may change within the solver's tolerance: the
 // stage sums are fused multiply-add chains over h-scaled weights, the
 // controller's powers go through the engine's exp and log (integer fixed
-// point), and the error norm's and the controller's divisions are
-// multiplications by the engine's reciprocal.  Everything else
+// point), and the divisions of the error norm, the controller, the initial
+// step size and the interpolation point are multiplications by the engine's
+// reciprocal.  Everything else
 // (controller logic, truncation, dense output, zero_every) computes the
 // reference's values exactly.  On 65,536 instances of the batched sirode
 // workload the solutions stay within 4e-13 relative of the reference's
@@ -110,6 +111,16 @@ struct state {
   int n_steps_accepted;
   int n_steps_rejected;
   int err;           // error code (0 = none)
+  // The dense-output record of the last accepted step is formed when it is
+  // needed (settle, dense_output).  Until then c1 holds y before the step,
+  // c2 its change and c3 the derivative before it; the stages are still in
+  // scratch (k3 .. k6, and the derivative after it in k2).  c4_set marks
+  // entries of c4 that interpolate_reset has written since.
+  bool pending;
+  unsigned c4_set;
+  // log(max(error, 1e-4)), when known
+  bool has_log_error;
+  double log_error;
 };
 
 template <int NV>
@@ -136,6 +147,14 @@ DUST2_HD double ref_max(double a, double b) {
   return (a < b) ? b : a;
 }
 
+// ref_max(|a|, |b|) with the comparison on the bits (a NaN counts as
+// larger than any number; the caller's result is then NaN either way).
+DUST2_HD double max_abs(double a, double b) {
+  const std::uint64_t ua = math::bits_of(a) & 0x7fffffffffffffffull;
+  const std::uint64_t ub = math::bits_of(b) & 0x7fffffffffffffffull;
+  return math::from_bits(ua < ub ? ub : ua);
+}
+
 DUST2_HD double clamp(double x, double lo, double hi) {
   return ref_max(ref_min(x, hi), lo);
 }
@@ -160,6 +179,17 @@ DUST2_HD double recip(double x) {
   return e - (1023 - 99) <= 198 ? math::rcp(x) : 1.0 / x;
 }
 
+// Systems whose state always has n_state_max entries may declare
+// `static constexpr bool fixed_n_state = true`.  The solver's loops over
+// variables then have no test of the number of variables: with one, the
+// compiler kept every stage sum of sirode's S, I, R and two case counts
+// (45 FP64 instructions a step) although the rhs reads S and I only.
+template <class T, class = void>
+struct has_fixed_n_state : std::false_type {};
+template <class T>
+struct has_fixed_n_state<T, std::void_t<decltype(T::fixed_n_state)>>
+  : std::integral_constant<bool, T::fixed_n_state> {};
+
 template <typename T, int NV>
 struct solver {
   const control_dev& ctl;
@@ -172,6 +202,14 @@ struct solver {
   int n_special = 0;
   // 1 / n_var for the error norm's mean
   double inv_n_var = 1.0 / n_var;
+  // the controller's constant logarithms
+  double log_safe = math::log(ctl.factor_safe);
+  double log_floor = math::log(1e-4);
+
+  // Whether entry i is one of the integrated variables.
+  DUST2_HD bool on(int i) const {
+    return has_fixed_n_state<T>::value || i < n_var;
+  }
 
   DUST2_HD void copy_special(const double* y, double* dst) {
 #pragma unroll
@@ -205,19 +243,19 @@ struct solver {
       b76 = h * A76;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      if (i < n_var) s.y_next[i] = std::fma(b21, k1[i], y[i]);
+      if (on(i)) s.y_next[i] = std::fma(b21, k1[i], y[i]);
     }
     rhs(t + C2 * h, s.y_next, s.k2);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      if (i < n_var) {
+      if (on(i)) {
         s.y_next[i] = std::fma(b32, s.k2[i], std::fma(b31, k1[i], y[i]));
       }
     }
     rhs(t + C3 * h, s.y_next, s.k3);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      if (i < n_var) {
+      if (on(i)) {
         double acc = std::fma(b41, k1[i], y[i]);
         acc = std::fma(b42, s.k2[i], acc);
         s.y_next[i] = std::fma(b43, s.k3[i], acc);
@@ -226,7 +264,7 @@ struct solver {
     rhs(t + C4 * h, s.y_next, s.k4);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      if (i < n_var) {
+      if (on(i)) {
         double acc = std::fma(b51, k1[i], y[i]);
         acc = std::fma(b52, s.k2[i], acc);
         acc = std::fma(b53, s.k3[i], acc);
@@ -236,7 +274,7 @@ struct solver {
     rhs(t + C5 * h, s.y_next, s.k5);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      if (i < n_var) {
+      if (on(i)) {
         double acc = std::fma(b61, k1[i], y[i]);
         acc = std::fma(b62, s.k2[i], acc);
         acc = std::fma(b63, s.k3[i], acc);
@@ -247,7 +285,7 @@ struct solver {
     rhs(t_next, s.y_stiff, s.k6);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      if (i < n_var) {
+      if (on(i)) {
         double acc = std::fma(b71, k1[i], y[i]);
         acc = std::fma(b73, s.k3[i], acc);
         acc = std::fma(b74, s.k4[i], acc);
@@ -256,61 +294,80 @@ struct solver {
       }
     }
     rhs(t_next, s.y_next, s.k2);
-    const double d1 = h * D1, d3 = h * D3, d4 = h * D4, d5 = h * D5,
-      d6 = h * D6, d7 = h * D7;
     const double e1 = h * E1, e3 = h * E3, e4 = h * E4, e5 = h * E5,
       e6 = h * E6, e7 = h * E7;
+    double err = 0.0;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      if (i < n_var) {
-        double acc = d1 * k1[i];
-        acc = std::fma(d3, s.k3[i], acc);
-        acc = std::fma(d4, s.k4[i], acc);
-        acc = std::fma(d5, s.k5[i], acc);
-        acc = std::fma(d6, s.k6[i], acc);
-        st.c5[i] = std::fma(d7, s.k2[i], acc);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      if (i < n_var) {
+      if (on(i)) {
         double acc = e1 * k1[i];
         acc = std::fma(e3, s.k3[i], acc);
         acc = std::fma(e4, s.k4[i], acc);
         acc = std::fma(e5, s.k5[i], acc);
         acc = std::fma(e6, s.k6[i], acc);
-        s.k4[i] = std::fma(e7, s.k2[i], acc);
-      }
-    }
-    double err = 0.0;
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      if (i < n_var) {
-        const double sk = s.k4[i] *
-          recip(std::fma(ctl.rtol, ref_max(fabs(y[i]), fabs(s.y_next[i])),
-                         ctl.atol));
+        acc = std::fma(e7, s.k2[i], acc);
+        const double sk = acc *
+          recip(std::fma(ctl.rtol, max_abs(y[i], s.y_next[i]), ctl.atol));
         err = std::fma(sk, sk, err);
       }
     }
     return sqrt(err * inv_n_var);
   }
 
+  // The record of an accepted step: what settle and dense_output need and
+  // the next trial step overwrites.  Forming c3, c4 and c5 of every entry
+  // at every step took 45 of a sirode step's 351 FP64 instructions, where
+  // only the entry being reset is ever interpolated.
   DUST2_HD void update_interpolation(double t, double h, const double* y,
                                      state<NV>& st, scratch<NV>& s) {
     st.t0 = t;
     st.t1 = t + h;
     st.h = h;
+    st.pending = true;
+    st.c4_set = 0;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      if (i < n_var) {
-        const double ydiff = s.y_next[i] - y[i];
-        const double bspl = std::fma(h, st.dydt[i], -ydiff);
+      if (on(i)) {
         st.c1[i] = y[i];
-        st.c2[i] = ydiff;
-        st.c3[i] = bspl;
-        st.c4[i] = std::fma(-h, s.k2[i], ydiff) - bspl;
+        st.c2[i] = s.y_next[i] - y[i];
+        st.c3[i] = st.dydt[i];
       }
     }
+  }
+
+  // Coefficients 3 to 5 of entry i of a pending record.
+  DUST2_HD void coefficients(int i, const state<NV>& st,
+                             const scratch<NV>& s, double* c3, double* c4,
+                             double* c5) const {
+    const double h = st.h;
+    const double k1 = st.c3[i];
+    *c3 = std::fma(h, k1, -st.c2[i]);
+    *c4 = (st.c4_set >> i) & 1 ? st.c4[i] :
+      std::fma(-h, s.k2[i], st.c2[i]) - *c3;
+    double acc = (h * D1) * k1;
+    acc = std::fma(h * D3, s.k3[i], acc);
+    acc = std::fma(h * D4, s.k4[i], acc);
+    acc = std::fma(h * D5, s.k5[i], acc);
+    acc = std::fma(h * D6, s.k6[i], acc);
+    *c5 = std::fma(h * D7, s.k2[i], acc);
+  }
+
+  // Complete the record, before it is stored.
+  DUST2_HD void settle(state<NV>& st, const scratch<NV>& s) const {
+    if (!st.pending) {
+      return;
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      if (on(i)) {
+        double c3, c4, c5;
+        coefficients(i, st, s, &c3, &c4, &c5);
+        st.c3[i] = c3;
+        st.c4[i] = c4;
+        st.c5[i] = c5;
+      }
+    }
+    st.pending = false;
   }
 
   DUST2_HD void record_step_time(double t) {
@@ -354,12 +411,11 @@ struct solver {
     // err^c / fac_old^beta / safe = exp(c log err - beta log fac_old -
     // log safe); log 0 = -Inf, and NaN and Inf propagate as through pow.
     const double log_err = math::log(err);
-    const double log_safe = math::log(ctl.factor_safe);
     if (err <= 1) {
       update_interpolation(t, h, y, st, s);
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
-        if (i < n_var) {
+        if (on(i)) {
           st.dydt[i] = s.k2[i];
           y[i] = s.y_next[i];
         }
@@ -367,15 +423,18 @@ struct solver {
       st.n_steps_accepted++;
       record_step_time(truncated ? t_end : t + h);
       if (!truncated) {
-        const double fac_old = ref_max(st.error, 1e-4);
+        // log fac_old is the last step's log err, or the floor's
+        const double log_old = st.has_log_error ? st.log_error :
+          math::log(ref_max(st.error, 1e-4));
         const double log_fac = std::fma(ctl.constant, log_err,
-                                        -ctl.beta * math::log(fac_old)) -
-          log_safe;
+                                        -ctl.beta * log_old) - log_safe;
         const double fac = clamp(math::exp(log_fac), ctl.facc2, ctl.facc1);
         const double h_new = h * recip(fac);
         const double h_max = reject ? h : ctl.step_size_max;
         st.step_size = ref_min(h_new, h_max);
         st.error = err;
+        st.log_error = err < 1e-4 ? log_floor : log_err;
+        st.has_log_error = true;
       }
       t = truncated ? t_end : t + h;
       return 1;
@@ -403,28 +462,34 @@ struct solver {
   // written into c4[0..] in index order (the reference uses c4 as its
   // scratch buffer, solver.hpp:456-458) and then subtracted from y.
   DUST2_HD void interpolate_reset(const zero_every_spec& z, int e,
-                                  double t_reset, double* y, state<NV>& st) {
-    const double u = (t_reset - st.t0) / st.h;
+                                  double t_reset, double* y, state<NV>& st,
+                                  const scratch<NV>& s) {
+    const double u = (t_reset - st.t0) * recip(st.h);
     const double v = 1 - u;
     int r = 0;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      if (i < n_var && z.has(e, i)) {
-        const double val = st.c1[i] + u * (st.c2[i] + v * (st.c3[i] + u *
-                                      (st.c4[i] + v * st.c5[i])));
+      if (on(i) && z.has(e, i)) {
+        double c3 = st.c3[i], c4 = st.c4[i], c5 = st.c5[i];
+        if (st.pending) {
+          coefficients(i, st, s, &c3, &c4, &c5);
+        }
+        const double val = st.c1[i] + u * (st.c2[i] + v * (c3 + u *
+                                                           (c4 + v * c5)));
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
           if (q == r) {
             st.c4[q] = val;
           }
         }
+        st.c4_set |= 1u << r;
         ++r;
       }
     }
     r = 0;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      if (i < n_var && z.has(e, i)) {
+      if (on(i) && z.has(e, i)) {
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
           if (q == r) {
@@ -437,26 +502,25 @@ struct solver {
   }
 
   DUST2_HD void apply_zero_every(double t, double* y, const zero_every_spec& z,
-                                 state<NV>& st) {
+                                 state<NV>& st, const scratch<NV>& s) {
     if (z.n == 0 || st.h == 0) {
       return;
     }
     for (int e = 0; e < z.n; ++e) {
       const double period = z.period[e];
-      const int n = static_cast<int>(math::floor_bits(div_period(t, period)));
-      const int m =
-        static_cast<int>(math::floor_bits(div_period(st.t0, period)));
+      const double n = math::floor_bits(div_period(t, period));
+      const double m = math::floor_bits(div_period(st.t0, period));
       if (n > m) {
         const double t_reset = n * period;
         if (t_reset == t) {
 #pragma unroll
           for (int i = 0; i < NV; ++i) {
-            if (i < n_var && z.has(e, i)) {
+            if (on(i) && z.has(e, i)) {
               y[i] = 0;
             }
           }
         } else {
-          interpolate_reset(z, e, t_reset, y, st);
+          interpolate_reset(z, e, t_reset, y, st, s);
         }
       }
     }
@@ -464,7 +528,7 @@ struct solver {
 
   DUST2_HD void apply_zero_every_final(double t, double* y,
                                        const zero_every_spec& z,
-                                       state<NV>& st) {
+                                       state<NV>& st, const scratch<NV>& s) {
     if (z.n == 0 || st.h == 0) {
       return;
     }
@@ -475,7 +539,7 @@ struct solver {
         const int m = static_cast<int>(ceil(div_period(st.t0, period)));
         if (n > m) {
           const double t_reset = (n - 1) * period;
-          interpolate_reset(z, e, t_reset, y, st);
+          interpolate_reset(z, e, t_reset, y, st, s);
         }
       }
     }
@@ -491,7 +555,7 @@ struct solver {
     }
     if (ctl.n_critical == 0) {
       while (t < t_end && st.err == 0) {
-        apply_zero_every(t, y, z, st);
+        apply_zero_every(t, y, z, st, s);
         t = step(t, t_end, y, st, s);
       }
     } else {
@@ -502,7 +566,7 @@ struct solver {
       double t_end_i = (tc == ctl.n_critical || ctl.critical[tc] >= t_end) ?
         t_end : ctl.critical[tc];
       while (t < t_end && st.err == 0) {
-        apply_zero_every(t, y, z, st);
+        apply_zero_every(t, y, z, st, s);
         t = step(t, t_end_i, y, st, s);
         if (t >= t_end_i && t < t_end) {
           ++tc;
@@ -512,7 +576,7 @@ struct solver {
       }
     }
     if (st.err == 0) {
-      apply_zero_every_final(t, y, z, st);
+      apply_zero_every_final(t, y, z, st, s);
     }
     return t;
   }
@@ -523,6 +587,7 @@ struct solver {
                            scratch<NV>& s) {
     st.step_size = 0;
     st.error = 0;
+    st.has_log_error = false;
     st.n_steps = 0;
     st.n_steps_accepted = 0;
     st.n_steps_rejected = 0;
@@ -531,8 +596,9 @@ struct solver {
     }
     record_step_time(t);
     double* f0 = st.dydt;
-    double* f1 = s.k3;
+    double* f1 = s.y_stiff;  // not the stages of a pending record
     double* y1 = s.y_next;
+    double inv_sk[NV];
     if (n_special > 0) {
       copy_special(y, y1);
     }
@@ -541,10 +607,12 @@ struct solver {
     double norm_y = 0.0;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      if (i < n_var) {
-        const double sk = ctl.atol + ctl.rtol * fabs(y[i]);
-        norm_f += square(f0[i] / sk);
-        norm_y += square(y[i] / sk);
+      if (on(i)) {
+        inv_sk[i] = recip(std::fma(ctl.rtol, fabs(y[i]), ctl.atol));
+        const double f = f0[i] * inv_sk[i];
+        const double g = y[i] * inv_sk[i];
+        norm_f = std::fma(f, f, norm_f);
+        norm_y = std::fma(g, g, norm_y);
       }
     }
     double h = (norm_f <= 1e-10 || norm_y <= 1e-10) ?
@@ -552,17 +620,17 @@ struct solver {
     h = ref_min(h, ctl.step_size_max);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      if (i < n_var) {
-        y1[i] = y[i] + h * f0[i];
+      if (on(i)) {
+        y1[i] = std::fma(h, f0[i], y[i]);
       }
     }
     rhs(t + h, y1, f1);
     double der2 = 0.0;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      if (i < n_var) {
-        const double sk = ctl.atol + ctl.rtol * fabs(y[i]);
-        der2 += square((f1[i] - f0[i]) / sk);
+      if (on(i)) {
+        const double f = (f1[i] - f0[i]) * inv_sk[i];
+        der2 = std::fma(f, f, der2);
       }
     }
     der2 = sqrt(der2) / h;
@@ -570,7 +638,7 @@ struct solver {
     const double der12 = ref_max(fabs(der2), sqrt(norm_f));
     const double h1 = (der12 <= 1e-15) ?
       ref_max(1e-6, fabs(h) * 1e-3) :
-      pow(0.01 / der12, 1.0 / order);
+      math::exp(math::log(0.01 / der12) / order);
     h = ref_min(100 * fabs(h), h1);
     if (!isfinite(h)) {
       st.err = ERR_ODE_INITIAL_STEP;

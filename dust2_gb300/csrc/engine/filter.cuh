@@ -204,8 +204,11 @@ __device__ __forceinline__ void step_compare_tile(
 // advance()), and compares its state as it stands, outputs not refreshed
 // (continuous/system.hpp:279-305).  The group reductions are
 // k_step_compare's.
+// (Registers as the solver needs them, 255 at most: the number of warps is
+// not what bounds it.)
 template <typename T>
-DUST2_PARTICLE_KERNEL(T) k_step_compare_mixed(
+__global__ void __launch_bounds__(default_tile_size<T>())
+k_step_compare_mixed(
     system_view<T> v, ode_view o, dopri5::control_dev ctl, filter_view f,
     double time0, double time, double dt, int initialise,
     const typename T::data_type* data, int n_groups_data) {
@@ -243,6 +246,7 @@ DUST2_PARTICLE_KERNEL(T) k_step_compare_mixed(
     const auto& d = data[n_groups_data == 1 ? 0 : tl.group];
     logw = T::compare_data(time, y, d, shared, internal, rng);
     store_state<T>(v, k, y);
+    sol.settle(st, s);
     store_ode<NV>(o, k, n_var, st);
     if (st.err != 0 || update_err != 0) {
       rng.err = st.err != 0 ? st.err : update_err;
@@ -447,8 +451,8 @@ public:
       allow_count_smem<T>(k_step_compare<T>);
       allow_count_smem<T>(k_step_compare_queue<T>);
       queue_.resize(std::max<std::size_t>(1, schedule_.size()));
-      set_shape(default_shape());
     }
+    set_shape(default_shape());
     // k_group: one warp per window of 32 chunks of the largest group
     int n_win = 1;
     for (int c : L.chunk_count) {
@@ -996,8 +1000,12 @@ public:
                                t.size() * sizeof(tile),
                                cudaMemcpyHostToDevice, sys_->stream()));
     n_step_tiles_ = static_cast<int>(t.size());
-    step_grid_ = sh.persistent ? persistent_grid(sh.block, n_step_tiles_) :
-      n_step_tiles_;
+    step_grid_ = n_step_tiles_;
+    if constexpr (!is_continuous<T>()) {
+      if (sh.persistent) {
+        step_grid_ = persistent_grid(sh.block, n_step_tiles_);
+      }
+    }
     shape_ = sh;
     graph_state_ptr_ = nullptr;  // force a re-capture
     DUST2_CUDA(cudaStreamSynchronize(sys_->stream()));
@@ -1220,7 +1228,7 @@ private:
     f.gflag = gflag_.data();
     if (timing_) {
       ensure_events();
-      record(ev_run_[0]);
+      this->record(ev_run_[0]);
     }
     k_filter_reset<<<n_blocks(G, 128), 128, 0, s>>>(f, G);
     if constexpr (!is_continuous<T>()) {
@@ -1236,22 +1244,28 @@ private:
                                            time_start_);
     double* cur = S.state_ptr();
     double* other = S.state_other_ptr();
+    ode_view record{}, record_other{};
+    if constexpr (is_continuous<T>()) {
+      record = owner_->view_ode();
+      record_other = owner_->view_ode_other();
+    }
     for (std::size_t i = 0; i < schedule_.size(); ++i) {
       const auto& st = schedule_[i];
       v.state = cur;
       if (timing_) {
-        record(ev_step_[2 * i]);
+        this->record(ev_step_[2 * i]);
       }
       if constexpr (is_continuous<T>()) {
-        k_step_compare_mixed<T><<<NT, TS, 0, s>>>(
-          v, owner_->view_ode(), owner_->control_dev(), f, st.t0,
+        v.tiles = step_tiles_.data();
+        k_step_compare_mixed<T><<<n_step_tiles_, shape_.block, 0, s>>>(
+          v, record, owner_->control_dev(), f, st.t0,
           st.t_compare, owner_->dt(), i == 0 ? 1 : 0,
           data_.data() + i * n_groups_data_, n_groups_data_);
       } else {
         launch_step(s, f, v.state, v.rng, st, i, queue_.data() + i);
       }
       if (timing_) {
-        record(ev_step_[2 * i + 1]);
+        this->record(ev_step_[2 * i + 1]);
       }
       if (fused_tail_) {
         k_tail_cluster<<<G * TAIL_CLUSTER, TAIL_BLOCK, 0, s>>>(
@@ -1262,19 +1276,21 @@ private:
         k_resample<<<NT, TS, 0, s>>>(f);
         k_fallback_counted(f, s);
         if (timing_) {
-          record(ev_reorder_[2 * i]);
+          this->record(ev_reorder_[2 * i]);
         }
         k_reorder<<<NT, TS, 0, s>>>(cur, other, L.stride, S.n_state(),
                                     L.tiles.empty() ? nullptr :
                                     S.tiles_dev(), offset_.data(),
                                     idx_.data(), mode_.data());
         if (timing_) {
-          record(ev_reorder_[2 * i + 1]);
+          this->record(ev_reorder_[2 * i + 1]);
         }
       }
       if constexpr (is_continuous<T>()) {
-        owner_->enqueue_reorder_record(S.tiles_dev(), NT, TS, offset_.data(),
-                                       idx_.data(), mode_.data(), s);
+        owner_->enqueue_reorder_record(record, record_other, S.tiles_dev(),
+                                       NT, TS, offset_.data(), idx_.data(),
+                                       mode_.data(), s);
+        std::swap(record, record_other);
       }
       std::swap(cur, other);
       const std::size_t stride = L.stride;
@@ -1300,9 +1316,14 @@ private:
                                  static_cast<std::size_t>(S.n_state()) *
                                  L.stride * sizeof(double),
                                  cudaMemcpyDeviceToDevice, s));
+      if constexpr (is_continuous<T>()) {
+        owner_->enqueue_reorder_record(record, record_other, S.tiles_dev(),
+                                       NT, TS, offset_.data(), nullptr,
+                                       nullptr, s);
+      }
     }
     if (timing_) {
-      record(ev_run_[1]);
+      this->record(ev_run_[1]);
     }
     DUST2_CUDA(cudaGetLastError());
   }

@@ -177,6 +177,7 @@ DUST2_PARTICLE_KERNEL(T) k_unfilter_ode(
     }
     refresh_output<T>(t, y, shared, internal);
     store_state<T>(v, k, y);
+    sol.settle(st, s);
     store_ode<NV>(o, k, n_var, st);
     ll[k] = acc;
     if (st.err != 0 || update_err != 0) {

@@ -31,6 +31,7 @@ struct malaria {
     real_type initial_Iv;
     real_type initial_Sv;
     real_type beta_volatility;
+    real_type rate;   // n_rates / tau
   };
   struct internal_state {};
   struct data_type {
@@ -76,6 +77,7 @@ struct malaria {
     s.bh = 0.05;
     s.bv = 0.05;
     s.mu = -math::log(0.9);
+    s.rate = s.n_rates / s.tau;
     return s;
   }
 
@@ -83,6 +85,7 @@ struct malaria {
     s.a = read_par_update<malaria>(pars, 0, s.a);
     s.r = read_par_update<malaria>(pars, 2, s.r);
     s.tau = read_par_update<malaria>(pars, 3, s.tau);
+    s.rate = s.n_rates / s.tau;
   }
 
   static std::vector<packing_entry> packing_state(const shared_state& s) {
@@ -129,7 +132,7 @@ struct malaria {
     const real_type beta = state[4 + n];
     const real_type foi_h = shared.a * shared.bh * Iv;
     const real_type foi_v = shared.a * shared.bv * Ih;
-    const real_type rate = n / shared.tau;
+    const real_type rate = shared.rate;
     state_deriv[4] = foi_v * Sv - rate * Ev[0] - shared.mu * Ev[0];
     for (int i = 1; i < n; ++i) {
       state_deriv[4 + i] = rate * Ev[i - 1] - rate * Ev[i] -

@@ -18,6 +18,7 @@ struct sirode {
     real_type I0;
     real_type beta;
     real_type gamma;
+    math::divisor by_N;
   };
   struct internal_state {};
   struct data_type {
@@ -26,6 +27,7 @@ struct sirode {
 
   static constexpr int n_state_max = 5;
   static constexpr int n_output = 0;
+  static constexpr bool fixed_n_state = true;
 
   static constexpr parameter_info parameters[] = {
     {"I0", 1, 10, false, false},
@@ -40,6 +42,7 @@ struct sirode {
     s.N = read_par<sirode>(pars, 1);
     s.beta = read_par<sirode>(pars, 2);
     s.gamma = read_par<sirode>(pars, 3);
+    s.by_N = math::divisor::of(s.N);
     return s;
   }
 
@@ -85,7 +88,7 @@ struct sirode {
                            real_type* state_deriv) {
     const auto S = state[0];
     const auto I = state[1];
-    const auto rate_SI = shared.beta * S * I / shared.N;
+    const auto rate_SI = math::divide(shared.beta * S * I, shared.by_N);
     const auto rate_IR = shared.gamma * I;
     state_deriv[0] = -rate_SI;
     state_deriv[1] = rate_SI - rate_IR;
