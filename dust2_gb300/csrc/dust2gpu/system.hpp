@@ -170,6 +170,15 @@ template <class T>
 struct has_adjoint<T, std::void_t<decltype(&T::adjoint_update)>>
   : std::true_type {};
 
+// An adjoint split into what depends on the state only (adjoint_prepare,
+// adjoint_compare_prepare) and the rest (adjoint_update_tape,
+// adjoint_compare_tape), with the same results.
+template <class T, class = void>
+struct has_adjoint_tape : std::false_type {};
+template <class T>
+struct has_adjoint_tape<T, std::void_t<typename T::adjoint_tape>>
+  : std::true_type {};
+
 template <class T, class = void>
 struct has_output : std::false_type {};
 template <class T>

@@ -107,8 +107,8 @@ struct sir {
     const auto R = state[2];
     const auto cases_cumul = state[3];
     const auto cases_inc = state[4];
-    const auto p_SI = 1 - math::exp(-shared.beta * I / shared.N * dt);
-    const auto p_IR = 1 - math::exp(-shared.gamma * dt);
+    const auto p_SI = p_infect(I, dt, shared);
+    const auto p_IR = p_recover(dt, shared);
     const auto n_SI = random::binomial(rng_state, S, p_SI);
     const auto n_IR = random::binomial(rng_state, I, p_IR);
     state_next[0] = S - n_SI;
@@ -116,6 +116,23 @@ struct sir {
     state_next[2] = R + n_IR;
     state_next[3] = cases_cumul + n_SI;
     state_next[4] = cases_inc + n_SI;
+  }
+
+  // x / N, 1 - exp(-beta I / N dt) and 1 - exp(-gamma dt), with what was
+  // prepared for dt where it was (the same values).
+  DUST2_HD static real_type over_N(real_type x, real_type dt,
+                                   const shared_state& shared) {
+    return shared.counts.prepared(dt) ?
+      math::divide(x, shared.counts.by_N) : x / shared.N;
+  }
+  DUST2_HD static real_type p_infect(real_type I, real_type dt,
+                                     const shared_state& shared) {
+    return 1 - math::exp(over_N(-shared.beta * I, dt, shared) * dt);
+  }
+  DUST2_HD static real_type p_recover(real_type dt,
+                                      const shared_state& shared) {
+    return shared.counts.prepared(dt) ? shared.counts.recover.p :
+      1 - math::exp(-shared.gamma * dt);
   }
 
   static void count_prepare(shared_state& s, real_type dt) {
@@ -174,14 +191,29 @@ struct sir {
     adjoint_next[7] = adjoint[7] + adj_I;
   }
 
-  DUST2_HD static void adjoint_update(real_type time, real_type dt,
-                                      const real_type* state,
-                                      const real_type* adjoint,
-                                      const shared_state& shared,
-                                      internal_state& internal,
-                                      real_type* adjoint_next) {
-    const auto S = state[0];
+  // What the step back needs of the state, apart from the adjoint: the
+  // engine forms it for several steps at once, one per lane.
+  struct adjoint_tape {
+    real_type S;
+    real_type I;
+    real_type p_SI;
+    real_type e_SI;
+  };
+
+  DUST2_HD static adjoint_tape adjoint_prepare(real_type dt,
+                                               const real_type* state,
+                                               const shared_state& shared) {
     const auto I = state[1];
+    return adjoint_tape{state[0], I, p_infect(I, dt, shared),
+                        math::exp(over_N(-shared.beta * I * dt, dt,
+                                         shared))};
+  }
+
+  DUST2_HD static void adjoint_update_tape(real_type dt,
+                                           const adjoint_tape& tape,
+                                           const real_type* adjoint,
+                                           const shared_state& shared,
+                                           real_type* adjoint_next) {
     const auto adj_S = adjoint[0];
     const auto adj_I = adjoint[1];
     const auto adj_R = adjoint[2];
@@ -190,22 +222,51 @@ struct sir {
     const auto adj_beta = adjoint[5];
     const auto adj_gamma = adjoint[6];
     const auto adj_I0 = adjoint[7];
-    const auto p_SI = 1 - math::exp(-shared.beta * I / shared.N * dt);
-    const auto p_IR = 1 - math::exp(-shared.gamma * dt);
+    const auto p_IR = p_recover(dt, shared);
     const auto adj_n_IR = -adj_I + adj_R;
     const auto adj_n_SI = adj_cases_inc + adj_cases_cumul + adj_I + -adj_S;
-    const auto adj_p_IR = adj_n_IR * I;
-    const auto adj_p_SI = adj_n_SI * S;
-    const auto e_SI = math::exp(-shared.beta * I * dt / shared.N);
-    adjoint_next[0] = adj_n_SI * p_SI + adj_S;
+    const auto adj_p_IR = adj_n_IR * tape.I;
+    const auto adj_p_SI = adj_n_SI * tape.S;
+    const auto exp_gamma = shared.counts.prepared(dt) ?
+      shared.counts.exp_gamma : math::exp(-shared.gamma);
+    adjoint_next[0] = adj_n_SI * tape.p_SI + adj_S;
     adjoint_next[1] = adj_n_IR * p_IR +
-      adj_p_SI * (shared.beta * dt) * e_SI / shared.N + adj_I;
+      over_N(adj_p_SI * (shared.beta * dt) * tape.e_SI, dt, shared) + adj_I;
     adjoint_next[2] = adj_R;
     adjoint_next[3] = adj_cases_cumul;
     adjoint_next[4] = adj_cases_inc;
-    adjoint_next[5] = adj_beta + adj_p_SI * I * dt * e_SI / shared.N;
-    adjoint_next[6] = adj_gamma + adj_p_IR * math::exp(-shared.gamma);
+    adjoint_next[5] = adj_beta +
+      over_N(adj_p_SI * tape.I * dt * tape.e_SI, dt, shared);
+    adjoint_next[6] = adj_gamma + adj_p_IR * exp_gamma;
     adjoint_next[7] = adj_I0;
+  }
+
+  DUST2_HD static void adjoint_update(real_type time, real_type dt,
+                                      const real_type* state,
+                                      const real_type* adjoint,
+                                      const shared_state& shared,
+                                      internal_state& internal,
+                                      real_type* adjoint_next) {
+    adjoint_update_tape(dt, adjoint_prepare(dt, state, shared), adjoint,
+                        shared, adjoint_next);
+  }
+
+  // The comparison's part: the derivative with respect to cases_inc.
+  DUST2_HD static real_type adjoint_compare_prepare(
+      const real_type* state, const data_type& data,
+      const shared_state& shared) {
+    const real_type noise = 1 / shared.exp_noise;
+    const real_type lambda = state[4] + noise;
+    return data.incidence / lambda - 1;
+  }
+
+  DUST2_HD static void adjoint_compare_tape(real_type tape,
+                                            const real_type* adjoint,
+                                            real_type* adjoint_next) {
+    for (int i = 0; i < 8; ++i) {
+      adjoint_next[i] = adjoint[i];
+    }
+    adjoint_next[4] = adjoint[4] + tape;
   }
 
   DUST2_HD static void adjoint_compare_data(real_type time,
@@ -215,14 +276,8 @@ struct sir {
                                             const shared_state& shared,
                                             internal_state& internal,
                                             real_type* adjoint_next) {
-    const real_type cases_inc = state[4];
-    const real_type noise = 1 / shared.exp_noise;
-    const real_type lambda = cases_inc + noise;
-    const real_type adj_lambda = data.incidence / lambda - 1;
-    for (int i = 0; i < 8; ++i) {
-      adjoint_next[i] = adjoint[i];
-    }
-    adjoint_next[4] = adjoint[4] + adj_lambda;
+    adjoint_compare_tape(adjoint_compare_prepare(state, data, shared),
+                         adjoint, adjoint_next);
   }
 };
 

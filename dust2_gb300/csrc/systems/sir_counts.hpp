@@ -14,18 +14,26 @@ struct sir_counts {
   std::uint64_t key_dt;
   std::uint64_t rate62;  // beta dt / N in units of 2^-62: 2^-32 relative
   random::count_prob recover;
+  math::divisor by_N;
+  double exp_gamma;      // exp(-gamma)
   bool ok;
 
   void prepare(double N, double beta, double gamma, double dt) {
     key_dt = math::bits_of(dt);
+    by_N = math::divisor::of(N);
+    exp_gamma = math::exp(-gamma);
     const double rate = beta * dt / N;
     recover = random::make_count_prob(1 - math::exp(-gamma * dt));
     ok = recover.ok && N > 0 && rate >= 0x1p-30 && rate < 1;
     rate62 = ok ? static_cast<std::uint64_t>(std::ldexp(rate, 62)) : 0;
   }
 
+  // Prepared for this dt; ready: and the counts can be stepped.
+  DUST2_HD bool prepared(double dt) const {
+    return key_dt == math::bits_of(dt);
+  }
   DUST2_HD bool ready(double dt) const {
-    return ok && key_dt == math::bits_of(dt);
+    return ok && prepared(dt);
   }
 
   // I < 2^24 and rate < 1: a hazard of 4 or more would wrap, so it is
