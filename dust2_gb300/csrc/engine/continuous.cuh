@@ -58,6 +58,13 @@ struct ode_view {
 };
 
 template <int NV>
+__device__ __forceinline__ void load_ode_scalars(const ode_view& o, int k,
+                                                 dopri5::state<NV>& st);
+template <int NV>
+__device__ __forceinline__ void store_ode_scalars(
+    const ode_view& o, int k, const dopri5::state<NV>& st);
+
+template <int NV>
 __device__ __forceinline__ void load_ode(const ode_view& o, int k, int n_var,
                                          dopri5::state<NV>& st) {
   const long S = o.stride;
@@ -72,6 +79,13 @@ __device__ __forceinline__ void load_ode(const ode_view& o, int k, int n_var,
       st.c5[i] = o.c[(4 * NV + i) * S + k];
     }
   }
+  load_ode_scalars(o, k, st);
+}
+
+// The entries of a solver record that do not belong to a variable.
+template <int NV>
+__device__ __forceinline__ void load_ode_scalars(const ode_view& o, int k,
+                                                 dopri5::state<NV>& st) {
   st.t0 = o.t0[k];
   st.t1 = o.t1[k];
   st.h = o.h[k];
@@ -102,6 +116,12 @@ __device__ __forceinline__ void store_ode(const ode_view& o, int k, int n_var,
       o.c[(4 * NV + i) * S + k] = st.c5[i];
     }
   }
+  store_ode_scalars(o, k, st);
+}
+
+template <int NV>
+__device__ __forceinline__ void store_ode_scalars(
+    const ode_view& o, int k, const dopri5::state<NV>& st) {
   o.t0[k] = st.t0;
   o.t1[k] = st.t1;
   o.h[k] = st.h;

@@ -190,6 +190,15 @@ template <class T>
 struct has_fixed_n_state<T, std::void_t<decltype(T::fixed_n_state)>>
   : std::integral_constant<bool, T::fixed_n_state> {};
 
+// A system whose variables are shared out over lanes (each integrates its
+// own) sums the error norms over them: T::lane_sum(internal, x), the same
+// value in every lane.
+template <class T, class = void>
+struct has_lane_sum : std::false_type {};
+template <class T>
+struct has_lane_sum<T, std::void_t<decltype(&T::lane_sum)>>
+  : std::true_type {};
+
 template <typename T, int NV>
 struct solver {
   const control_dev& ctl;
@@ -209,6 +218,14 @@ struct solver {
   // Whether entry i is one of the integrated variables.
   DUST2_HD bool on(int i) const {
     return has_fixed_n_state<T>::value || i < n_var;
+  }
+
+  DUST2_HD double total(double x) const {
+    if constexpr (has_lane_sum<T>::value) {
+      return T::lane_sum(internal, x);
+    } else {
+      return x;
+    }
   }
 
   DUST2_HD void copy_special(const double* y, double* dst) {
@@ -311,7 +328,7 @@ struct solver {
         err = std::fma(sk, sk, err);
       }
     }
-    return sqrt(err * inv_n_var);
+    return sqrt(total(err) * inv_n_var);
   }
 
   // The record of an accepted step: what settle and dense_output need and
@@ -615,6 +632,8 @@ struct solver {
         norm_y = std::fma(g, g, norm_y);
       }
     }
+    norm_f = total(norm_f);
+    norm_y = total(norm_y);
     double h = (norm_f <= 1e-10 || norm_y <= 1e-10) ?
       1e-6 : sqrt(norm_y / norm_f) * 0.01;
     h = ref_min(h, ctl.step_size_max);
@@ -633,7 +652,7 @@ struct solver {
         der2 = std::fma(f, f, der2);
       }
     }
-    der2 = sqrt(der2) / h;
+    der2 = sqrt(total(der2)) / h;
     const double order = 5;
     const double der12 = ref_max(fabs(der2), sqrt(norm_f));
     const double h1 = (der12 <= 1e-15) ?

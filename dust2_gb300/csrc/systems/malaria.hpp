@@ -158,6 +158,92 @@ struct malaria {
       random::normal(rng_state, 0, shared.beta_volatility));
   }
 
+#if defined(__CUDACC__)
+  // The same equations with a particle's variables shared out over L lanes,
+  // V consecutive ones each (the vectors' Ev chain then needs one value of
+  // the lane before).  Every derivative is x y - a s - b s with the terms of
+  // rhs in their order, or x y - a s; entries past the last are 0.
+  template <int L>
+  struct lanes {
+    using shared_state = malaria::shared_state;
+    struct internal_state {
+      int lane;
+      unsigned mask;   // the particle's lanes of the warp
+      int n;           // n_rates
+      real_type beta;  // the special entry
+    };
+    static constexpr int V = (4 + n_rates_max + L - 1) / L;
+    static constexpr bool fixed_n_state = true;
+
+    template <int I>
+    __device__ static real_type get(const internal_state& in,
+                                    const real_type* y) {
+      return __shfl_sync(in.mask, y[I % V], I / V, L);
+    }
+
+    __device__ static real_type lane_sum(const internal_state& in,
+                                         real_type x) {
+#pragma unroll
+      for (int off = L / 2; off > 0; off >>= 1) {
+        x = x + __shfl_xor_sync(in.mask, x, off, L);
+      }
+      return x;
+    }
+
+    __device__ static void rhs(real_type time, const real_type* y,
+                               const shared_state& shared,
+                               const internal_state& in,
+                               real_type* state_deriv) {
+      const real_type Sh = get<0>(in, y);
+      const real_type Ih = get<1>(in, y);
+      const real_type Sv = get<2>(in, y);
+      const real_type Iv = get<3>(in, y);
+      const real_type before = __shfl_up_sync(in.mask, y[V - 1], 1, L);
+      real_type last = y[0];
+#pragma unroll
+      for (int v = 1; v < V; ++v) {
+        last = v == (3 + in.n) % V ? y[v] : last;
+      }
+      last = __shfl_sync(in.mask, last, (3 + in.n) / V, L);
+      const real_type foi_h = shared.a * shared.bh * Iv;
+      const real_type foi_v = shared.a * shared.bv * Ih;
+      const real_type rate = shared.rate;
+      const real_type mu = shared.mu;
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const int i = in.lane * V + v;
+        // Ev[1], Ev[2], ...
+        real_type x = rate, s = v > 0 ? y[v > 0 ? v - 1 : 0] : before;
+        real_type a = rate, b = mu;
+        bool two = true;
+        if (i == 0) {
+          x = shared.r, s = Ih, a = foi_h, two = false;
+        } else if (i == 1) {
+          x = foi_h, s = Sh, a = shared.r, two = false;
+        } else if (i == 2) {
+          x = in.beta, s = shared.initial_Sv, a = foi_v;
+        } else if (i == 3) {
+          x = rate, s = last, a = mu, two = false;
+        } else if (i == 4) {
+          x = foi_v, s = Sv;
+        } else if (i >= 4 + in.n) {
+          x = 0, s = 0, a = 0, b = 0;
+        }
+        const real_type d = x * s - a * y[v];
+        state_deriv[v] = two ? d - b * y[v] : d;
+      }
+    }
+
+    // update() on the special entry alone.
+    __device__ static real_type update_special(
+        real_type dt, real_type beta, const shared_state& shared,
+        rng_state_type& rng_state) {
+      return beta * math::exp(
+        random::normal(rng_state, 0, shared.beta_volatility));
+    }
+  };
+#endif
+
   DUST2_HD static real_type compare_data(const real_type time,
                                          const real_type* state,
                                          const data_type& data,
