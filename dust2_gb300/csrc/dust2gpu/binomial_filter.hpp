@@ -174,7 +174,6 @@ DUST2_HD prob make_prob(double p) {
 // certain when U is farther than that from F(x) on both sides.  (With
 // n p < 10, x > 40 has probability below 1e-12.)  Returns x, or -1.
 DUST2_HD float inversion(rng_state& rng, float n, const prob& q, float t) {
-  const rng_state keep = rng;
   const float u =
     static_cast<float>(static_cast<std::uint32_t>(next(rng) >> 32)) *
     0x1p-32f;
@@ -194,9 +193,7 @@ DUST2_HD float inversion(rng_state& rng, float n, const prob& q, float t) {
   if (u < lower) {
     return x;
   }
-  for (int w = 0; w < 4; ++w) {
-    rng.state[w] = keep.state[w];
-  }
+  previous(rng.state);
   return -1.0f;
 }
 
@@ -282,9 +279,10 @@ DUST2_HD float deviance_near(float m, float d) {
 //     -[D(k) - D(m)] + 1/2 log(h(m) h(n - m) / (h(k) h(n - k))),
 //     D(x) = deviance(x, n p) + deviance(n - x, n q)
 //   (log x! by h; the linear terms of the two deviances cancel), which
-//   has no large terms: 112 e D(k) + 20 e D(m) + 30 e, and 2 |k - n p|
-//   rel.  Where (n + 1) p rounds to the other side of an integer, f(m)
-//   is the same to 2^-24.
+//   has no large terms: 112 e D(k) + 20 e D(m) + 30 e, 2 |k - n p| rel,
+//   and for the two logarithms of the h (at most 48 in base 2) 4 e of the
+//   first and 120 e.  Where (n + 1) p rounds to the other side of an
+//   integer, f(m) is the same to 2^-24.
 // Returns k, or -1 when undecided (the generator is then at the undecided
 // attempt's first uniform).
 DUST2_HD float btrs(rng_state& rng, float n, const prob& q, float np) {
@@ -299,10 +297,28 @@ DUST2_HD float btrs(rng_state& rng, float n, const prob& q, float np) {
   const float b = std::fmaf(2.53f, spq, 1.15f);
   const float a = std::fmaf(0.01f, q.p, std::fmaf(0.0248f, b, -0.0873f));
   const float inv_b = rcp32(b);
-  const float v_r = std::fmaf(-4.2f, inv_b, 0.92f);
+  // v's bounds, in units of 2^-32 as v is
+  const float v_r = std::fmaf(-4.2f * 0x1p32f, inv_b, 0.92f * 0x1p32f);
+  const float v_low = v_r - 12 * E * 0x1p32f;
+  const float v_high = v_r + 12 * E * 0x1p32f;
   const float y_band = std::fmaf(np, q.rel, std::fmaf(b, E, 4 * E));
+  const float a2 = 2.0f * 0x1p32f * a;
+  const float b_band = 14 * E * b;
+  // the acceptance test's terms that do not depend on the candidate: alpha
+  // 2^-32, and -D(m) - 1/2 log(h(m) h(n - m))
+  const float alpha = std::fmaf(5.1f, inv_b, 2.83f) * spq * 0x1p-32f;
+  const float nq = n - np;
+  const float off = 0.5f - cf;
+  float mode;
+  {
+    const float fm = std::floor(q.p - off);
+    const float m = ci + fm;
+    const float dm = fm + off;
+    mode = std::fmaf(
+      -0.5f * LN2, lg2_32(stirling_h10(m) * stirling_h10(n - m)),
+      -(deviance_near(np, dm) + deviance_near(nq, -dm)));
+  }
   for (int attempt = 0; attempt < 1000; ++attempt) {
-    const rng_state keep = rng;
     const std::uint32_t hu = static_cast<std::uint32_t>(next(rng) >> 32);
     const std::uint32_t hv = static_cast<std::uint32_t>(next(rng) >> 32);
     // u = U - 1/2 in units of 2^-32 (cut), us = 1/2 - |u|
@@ -310,47 +326,38 @@ DUST2_HD float btrs(rng_state& rng, float n, const prob& q, float np) {
     const std::uint32_t ad = neg ? 0x80000000u - hu : hu - 0x80000000u;
     const std::uint32_t us = 0x80000000u - ad;
     const float au = static_cast<float>(ad) * 0x1p-32f;
-    const float inv_us = rcp32(static_cast<float>(us) * 0x1p-32f);
-    const float v = static_cast<float>(hv) * 0x1p-32f;
-    const float t = 2.0f * a * inv_us;
-    const float g = (t + b) * au;
-    const float y = cf + (neg ? -g : g);
+    const float inv_us = rcp32(static_cast<float>(us));  // 2^-32 / us
+    const float v = static_cast<float>(hv);
+    const float t = a2 * inv_us;
+    const float y = std::fmaf(t + b, neg ? -au : au, cf);
     const float band_y = std::fmaf(
-      au, std::fmaf(t, std::fmaf(inv_us, 0x1p-32f, 34 * E), 14 * E * b),
-      y_band);
+      au, std::fmaf(t, inv_us + 34 * E, b_band), y_band);
     const float fl = std::floor(y);
     if (std::fabs(y - fl - 0.5f) < 0.5f - band_y) {
       const float k = ci + fl;
       // 0.07 2^32 = 300647710.72
       const bool squeeze = us >= 300647712u;
-      if (squeeze && v < v_r - 12 * E) {
+      if (squeeze && v < v_low) {
         return k;
       }
-      if (us <= 300647709u || (squeeze && v > v_r + 12 * E)) {
+      if (us <= 300647709u || (squeeze && v > v_high)) {
         if (k < 0.0f || k > n) {
           continue;
         }
-        const float alpha = std::fmaf(5.1f, inv_b, 2.83f) * spq;
+        // a / us^2 = (a2 / 2) (2^32 / us) / us
         const float lhs =
-          lg2_32(v * alpha * rcp32(std::fmaf(a * inv_us, inv_us, b)));
-        const float nq = n - np;
-        const float off = 0.5f - cf;
-        const float fm = std::floor(q.p - off);
-        const float m = ci + fm;
+          lg2_32(v * alpha *
+                 rcp32(std::fmaf(0.5f * 0x1p32f * t, inv_us, b)));
         const float dk = fl + off;
-        const float dm = fm + off;
         const float d_k = deviance(k, np, dk) + deviance(n - k, nq, -dk);
-        const float d_m = deviance_near(np, dm) + deviance_near(nq, -dm);
-        const float lg_h =
-          lg2_32(stirling_h10(m) * stirling_h10(n - m) *
-                 rcp32(stirling_h(k) * stirling_h(n - k)));
+        const float lg_h = lg2_32(stirling_h(k) * stirling_h(n - k));
         // left side minus right side
-        const float diff = std::fmaf(LN2, std::fmaf(-0.5f, lg_h, lhs),
-                                     d_k - d_m);
-        const float cut = std::fmaf(2.0f, inv_us, rcp32(v)) * 0x1p-32f;
+        const float diff = std::fmaf(LN2, std::fmaf(0.5f, lg_h, lhs),
+                                     d_k + mode);
+        const float cut = std::fmaf(2.0f, inv_us, rcp32(v));
         const float band = std::fmaf(
           112 * E, d_k, std::fmaf(4 * E, std::fabs(lhs) + std::fabs(lg_h),
-                                  128 * E + cut)) +
+                                  224 * E + cut)) +
           2.0f * q.rel * std::fabs(dk);
         if (diff < -band) {
           return k;
@@ -360,9 +367,8 @@ DUST2_HD float btrs(rng_state& rng, float n, const prob& q, float np) {
         }
       }
     }
-    for (int w = 0; w < 4; ++w) {
-      rng.state[w] = keep.state[w];
-    }
+    previous(rng.state);
+    previous(rng.state);
     return -1.0f;
   }
   return -1.0f;

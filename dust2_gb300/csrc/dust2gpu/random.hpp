@@ -74,6 +74,19 @@ DUST2_HD std::uint64_t next(std::uint64_t* s) {
   return result;
 }
 
+// The state before the last next(): the linear engine is invertible
+// (s1 + (s1 << 17) over GF(2) is undone by its series).
+DUST2_HD void previous(std::uint64_t* s) {
+  const std::uint64_t s3 = (s[3] >> 45) | (s[3] << 19);
+  const std::uint64_t z = s[1] ^ s[2];
+  const std::uint64_t s1 = z ^ (z << 17) ^ (z << 34) ^ (z << 51);
+  const std::uint64_t s2 = s[1] ^ s1;
+  s[0] = s[0] ^ s3;
+  s[1] = s1;
+  s[2] = s2 ^ s[0];
+  s[3] = s3 ^ s1;
+}
+
 DUST2_HD std::uint64_t next(rng_state& s) {
   return next(s.state);
 }
