@@ -576,7 +576,7 @@ public:
     auto s = base_.stream();
     const int S = L.stride;
     auto move = [&](double* a, int n_rows) {
-      k_reorder<<<L.n_tiles(), L.tile_size, 0, s>>>(
+      k_reorder<<<reorder_grid(L.n_tiles(), n_rows), L.tile_size, 0, s>>>(
         a, other_.data(), S, n_rows, base_.tiles_dev(),
         base_.group_offsets_dev(), idx.data(), nullptr);
       DUST2_CUDA(cudaMemcpyAsync(a, other_.data(),

@@ -852,7 +852,8 @@ public:
     DUST2_CUDA(cudaMemcpyAsync(idx.data(), index,
                                layout_.n_total * sizeof(int),
                                cudaMemcpyHostToDevice, stream_));
-    k_reorder<<<layout_.n_tiles(), layout_.tile_size, 0, stream_>>>(
+    k_reorder<<<reorder_grid(layout_.n_tiles(), n_state_),
+                layout_.tile_size, 0, stream_>>>(
       state_.data(), state_other_.data(), layout_.stride, n_state_,
       tiles_.data(), offsets_dev_.data(), idx.data(), nullptr);
     DUST2_CUDA(cudaGetLastError());

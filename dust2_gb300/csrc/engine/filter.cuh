@@ -42,8 +42,8 @@
 // log-likelihood uses the parallel total; it matches the serial one to
 // better than n u relative (u = 2^-53).
 //
-// When every group has at most 1024 particles, steps 2-6 run as one
-// launch, k_tail_cluster (a cluster of blocks per group), with the same
+// When every group has at most 1024 particles (4096, for few groups), steps
+// 2-6 run as one launch, k_tail_cluster (a cluster of blocks per group), with the same
 // results.
 //
 // The whole sequence for all data times is captured once into a CUDA
@@ -472,12 +472,22 @@ __global__ void k_resample(filter_view f);
 // Block size of k_fallback_count (any multiple of 32 up to 1024 works).
 constexpr int FALLBACK_THREADS = 1024;
 // The one-launch tail: a cluster of TAIL_CLUSTER blocks of TAIL_BLOCK
-// threads per group, for groups of at most TAIL_MAX_PARTICLES.
+// threads per group, for groups of at most 8 x 128 particles; of
+// TAIL_BLOCK_LARGE threads for groups of at most 8 x 512, while two blocks
+// per SM hold all groups (more groups keep the device busy as separate
+// kernels).
 constexpr int TAIL_CLUSTER = 8;
 constexpr int TAIL_BLOCK = 128;
-constexpr int TAIL_MAX_PARTICLES = TAIL_CLUSTER * TAIL_BLOCK;
+constexpr int TAIL_BLOCK_LARGE = 512;
+// It moves the state of at most this many entries per particle; longer ones
+// are moved by k_reorder, on the whole device (3001 SEIR particles, 96
+// entries: 57 us for the tail with the move, 18 without).
+constexpr int TAIL_STATE = 8;
 __global__ void k_tail_cluster(filter_view f, int* count, const double* src,
                                double* dst, int stride, int n_state);
+__global__ void k_tail_cluster_large(filter_view f, int* count,
+                                     const double* src, double* dst,
+                                     int stride, int n_state);
 __global__ void k_save_history(const double* state, int stride,
                                const int* index_state, int n_save,
                                const tile* tiles, const int* active,
@@ -635,7 +645,11 @@ public:
     for (int n : sys_->layout().n_particles) {
       n_max = std::max(n_max, n);
     }
-    fused_tail_ = fused && n_max <= TAIL_MAX_PARTICLES;
+    const int G = sys_->layout().n_groups;
+    tail_block_ = n_max <= TAIL_CLUSTER * TAIL_BLOCK ? TAIL_BLOCK :
+      n_max <= TAIL_CLUSTER * TAIL_BLOCK_LARGE &&
+      G * TAIL_CLUSTER <= 2 * n_sms() ? TAIL_BLOCK_LARGE : 0;
+    fused_tail_ = fused && tail_block_ > 0;
     graph_state_ptr_ = nullptr;  // force a re-capture
   }
 
@@ -1425,21 +1439,25 @@ private:
         this->record(ev_step_[2 * i + 1]);
       }
       if (fused_tail_) {
-        k_tail_cluster<<<G * TAIL_CLUSTER, TAIL_BLOCK, 0, s>>>(
-          f, fallback_count_.data(), cur, other, L.stride, S.n_state());
+        (tail_block_ == TAIL_BLOCK ? k_tail_cluster : k_tail_cluster_large)
+          <<<G * TAIL_CLUSTER, tail_block_, 0, s>>>(
+            f, fallback_count_.data(), cur, other, L.stride,
+            S.n_state() <= TAIL_STATE ? S.n_state() : 0);
       } else {
         k_weights<<<NT, TS, 0, s>>>(f);
         k_group<<<G, group_threads_, 0, s>>>(f, G);
         k_resample<<<NT, TS, 0, s>>>(f);
         k_fallback_counted(f, s);
-        if (timing_) {
+      }
+      if (!fused_tail_ || S.n_state() > TAIL_STATE) {
+        if (timing_ && !fused_tail_) {
           this->record(ev_reorder_[2 * i]);
         }
-        k_reorder<<<NT, TS, 0, s>>>(cur, other, L.stride, S.n_state(),
-                                    L.tiles.empty() ? nullptr :
-                                    S.tiles_dev(), offset_.data(),
-                                    idx_.data(), mode_.data());
-        if (timing_) {
+        k_reorder<<<reorder_grid(NT, S.n_state()), TS, 0, s>>>(
+          cur, other, L.stride, S.n_state(),
+          L.tiles.empty() ? nullptr : S.tiles_dev(), offset_.data(),
+          idx_.data(), mode_.data());
+        if (timing_ && !fused_tail_) {
           this->record(ev_reorder_[2 * i + 1]);
         }
       }
@@ -1579,6 +1597,7 @@ private:
   bool use_graph_ = true;
   bool mixed_lanes_ = false;  // k_step_compare_lanes
   bool fused_tail_ = false;  // k_tail_cluster instead of separate kernels
+  int tail_block_ = 0;       // its block size for these groups (0: none)
   int group_threads_ = 32;   // block size of k_group
   bool pending_ = false;
   bool capturing_ = false;

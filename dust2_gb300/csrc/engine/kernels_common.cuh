@@ -6,6 +6,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 
@@ -120,10 +121,19 @@ static __global__ void k_reorder(const double* __restrict__ src,
   const int k = tl.start + threadIdx.x;
   const bool move = group_mode == nullptr || group_mode[tl.group] != 0;
   const int from = move ? group_offset[tl.group] + index[k] : k;
-  for (int s = 0; s < n_state; ++s) {
+#pragma unroll 4
+  for (int s = blockIdx.y; s < n_state; s += gridDim.y) {
     dst[static_cast<long>(s) * stride + k] =
       src[static_cast<long>(s) * stride + from];
   }
+}
+
+// Its grid: the state entries are shared out over the second dimension
+// while the tiles are few (a thread's loads are served one latency after
+// another: 24 tiles of 96 entries took 17 us).
+inline dim3 reorder_grid(int n_tiles, int n_state) {
+  const int rows = std::min(n_state, std::max(1, 2048 / std::max(1, n_tiles)));
+  return dim3(n_tiles, rows);
 }
 
 inline int n_blocks(long n, int block) {

@@ -1000,7 +1000,7 @@ private:
     k_resample<<<NT, TS, 0, s>>>(f);
     k_fallback_count<<<S, FALLBACK_THREADS, 0, s>>>(f,
                                                     fallback_count_.data());
-    k_reorder_active<<<NT, TS, 0, s>>>(cur(), other(), cap_particles_,
+    k_reorder_active<<<reorder_grid(NT, n_state_), TS, 0, s>>>(cur(), other(), cap_particles_,
                                        n_state_, tiles_.data(),
                                        active_.data(), offset_.data(),
                                        idx_.data(), mode_.data());

@@ -131,15 +131,6 @@ __device__ void group_finish(const filter_view& f, int g, double tot,
   f.gflag[g] = (mode == MODE_RESAMPLE && *f.force_serial) ? 1 : 0;
 }
 
-// One warp of a running group: chunk offsets, then group_finish.
-__device__ void group_update(const filter_view& f, int g, int lane) {
-  const double tot = group_has_sum(f, g) ?
-    group_chunk_offsets(f, g, lane) : 0.0;
-  if (lane == 0) {
-    group_finish(f, g, tot, draw_group_uniform(f, g));
-  }
-}
-
 // group_chunk_offsets with the whole block: its warps scan windows of 32
 // chunks at once, and the first one scans the totals of 32 windows (a carry
 // beyond them), where the one-warp loop adds them one after another.  The
@@ -321,7 +312,7 @@ __device__ int resample_index(const search_view& sv, int i, int* flag) {
       static_cast<std::int64_t>(math::bits_of(q));
   }
   if (!ok) {
-    atomicOr(flag, 1);
+    *flag = 1;  // by any number of threads
   }
   return m;
 }
@@ -483,7 +474,8 @@ __device__ double exact_running_sums(const double* w, double* ser, int n) {
 }
 
 // The whole block resamples group g serially and counts it.
-__device__ void serial_fallback(const filter_view& f, int g, int* count) {
+__device__ void serial_fallback(const filter_view& f, int g, double u,
+                                int* count) {
   __shared__ double total;
   const int n = f.n_particles[g];
   const double* w = f.ew + f.offset[g];
@@ -497,7 +489,6 @@ __device__ void serial_fallback(const filter_view& f, int g, int* count) {
   }
   __syncthreads();
   const double tot = total;
-  const double u = f.gu[g];
   const double uu0 = tot * u / n;
   const double du = tot / n;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -521,130 +512,221 @@ k_fallback_count(filter_view f, int* count) {
   if (!f.active[g] || f.mode[g] != MODE_RESAMPLE || !f.gflag[g]) {
     return;
   }
-  serial_fallback(f, g, count);
+  serial_fallback(f, g, f.gu[g], count);
 }
 
-// The tail of an observation for groups of at most TAIL_MAX_PARTICLES
+// chunk_offsets of a group of at most 32 W chunks by one warp, into shared
+// memory: the sums of group_chunk_offsets_block, in its structure (a scan
+// per window of 32 chunks, one of the window totals).  Returns the total.
+template <int W>
+__device__ __forceinline__ double chunk_offsets_warp(const double* sums,
+                                                     int nc, double* s_off,
+                                                     double* s_end) {
+  const int lane = threadIdx.x & 31;
+  double v[W], excl[W];
+  double win = 0;  // lane j: total of window j
+#pragma unroll
+  for (int j = 0; j < W; ++j) {
+    const int c = 32 * j + lane;
+    v[j] = c < nc ? sums[c] : 0.0;
+  }
+#pragma unroll
+  for (int j = 0; j < W; ++j) {
+    const double incl = warp_inclusive_scan(v[j]);
+    excl[j] = __shfl_up_sync(0xffffffffu, incl, 1);
+    if (lane == 0) {
+      excl[j] = 0;
+    }
+    const double total = __shfl_sync(0xffffffffu, incl, 31);
+    win = lane == j ? total : win;
+  }
+  double before = 0;
+  if constexpr (W > 1) {
+    win = warp_inclusive_scan(win);
+    before = __shfl_up_sync(0xffffffffu, win, 1);
+    if (lane == 0) {
+      before = 0;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < W; ++j) {
+    const int c = 32 * j + lane;
+    const double off = W > 1 ?
+      __shfl_sync(0xffffffffu, before, j) + excl[j] : excl[j];
+    if (c < nc) {
+      s_off[c] = off;
+      s_end[c] = off + v[j];
+    }
+  }
+  return __shfl_sync(0xffffffffu, win, W > 1 ? 31 : 0);
+}
+
+// The tail of an observation for groups of at most TAIL_CLUSTER * BLOCK
 // particles, as one launch: k_weights, k_group, k_resample,
-// k_fallback_count and k_reorder.  Each group is a cluster of
-// TAIL_CLUSTER blocks (warp w of block r holds the group's chunk
-// 4r + w), so the FP64 work of the group is spread over the FP64 units of
-// TAIL_CLUSTER SMs, one warp per SM partition, and the phases are
-// separated by cluster barriers, whose release/acquire semantics make the
-// global writes of one phase visible to the next.  Every value is
-// computed by the same device functions in the same order as by the
-// separate kernels, so the results are the same bits.  To shorten the
-// chain of dependent loads, the group's filter draw is taken before the
-// weights are summed, and each block searches shared-memory copies of the
-// group's prefix sums.  Every block of a running group takes all four
-// barriers whatever the data (the fourth as arrive and wait around the
-// state copy when no serial fallback runs; that choice is the same in
-// every block), so no barrier can wait for a block that has left.  The
-// state of every group moves from src to dst (in place for groups that
-// keep their particles), as k_reorder does.
-__global__ void __cluster_dims__(TAIL_CLUSTER, 1, 1)
-__launch_bounds__(TAIL_BLOCK)
-k_tail_cluster(filter_view f, int* count, const double* __restrict__ src,
-               double* __restrict__ dst, int stride, int n_state) {
-  __shared__ int flag;  // ambiguous decisions, used in block rank 0
-  // copies of the group's search arrays (n <= TAIL_MAX_PARTICLES)
-  __shared__ double s_end[TAIL_MAX_PARTICLES / 32];
-  __shared__ double s_off[TAIL_MAX_PARTICLES / 32];
-  __shared__ double s_pre[TAIL_MAX_PARTICLES];
+// k_fallback_count and k_reorder.  Each group is a cluster of TAIL_CLUSTER
+// blocks (warp w of block r holds the group's chunk r BLOCK / 32 + w), so
+// the FP64 work of the group is spread over the FP64 units of TAIL_CLUSTER
+// SMs.  Every value is computed by the operations of the separate kernels
+// in their structure, so the results are the same bits.
+//
+// What bounds it is the chain of dependent loads, FP64 sums and barriers.
+// So there is one cluster barrier before the search, after which every
+// block scans the group's chunk totals for itself, and one after it; ambiguous decisions set a flag in every block's shared
+// memory, and the state is moved before the last barrier is waited for (and
+// again if the group turns out to need the serial algorithm).  One block
+// records the group's sums, generator and log-likelihood, whose logarithm
+// it takes while the others search.  Groups of 1000 particles: 12.0 us an
+// observation (15.2 with four barriers around one block's sums).
+// Every block of a running group takes both barriers whatever the data, and
+// the third exactly when its flag, the same in every block, is set.
+template <int BLOCK>
+__device__ __forceinline__ void tail_cluster(
+    const filter_view& f, int* count, const double* __restrict__ src,
+    double* __restrict__ dst, int stride, int n_state) {
+  constexpr int MAX = TAIL_CLUSTER * BLOCK;
+  __shared__ int flag;  // some decision of the group is ambiguous
+  __shared__ double s_end[MAX / 32];
+  __shared__ double s_off[MAX / 32];
+  __shared__ double s_pre[MAX];
+  __shared__ double s_total;
+  __shared__ double s_mean;
+  __shared__ group_uniform s_draw;
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   const int g = blockIdx.x / TAIL_CLUSTER;
   const int rank = static_cast<int>(cluster.block_rank());
-  const int i = rank * TAIL_BLOCK + static_cast<int>(threadIdx.x);
+  const int i = rank * BLOCK + static_cast<int>(threadIdx.x);
   const bool active = f.active[g] != 0;
   const int n = f.n_particles[g];
   const int base = f.offset[g];
   const int k = base + i;
   int from = k;  // the source of this particle's state
-  bool arrived = false;  // barrier 4 arrived on, still to be waited for
-  if (active) {
-    const bool summed = group_has_sum(f, g);
-    group_uniform draw{};
-    if (rank == 0 && threadIdx.x == 0) {
-      flag = 0;
-      draw = draw_group_uniform(f, g);  // independent of the weights
-    }
-    if (summed && 32 * (i >> 5) < n) {
-      const bool valid = i < n;
-      const double e =
-        valid ? scaled_weight(f, k, ordered_value(f.gkey[g])) : 0.0;
-      const double incl = warp_inclusive_scan(e);
-      if (valid) {
-        f.ew[k] = e;
-        f.pre[k] = incl;
-      }
-      if ((i & 31) == 31) {
-        f.chunk_sum[f.chunk_first[g] + (i >> 5)] = incl;
+  auto move_state = [&] {
+    if (i < n) {
+#pragma unroll 8
+      for (int s = 0; s < n_state; ++s) {
+        dst[static_cast<long>(s) * stride + k] =
+          src[static_cast<long>(s) * stride + from];
       }
     }
-    cluster.sync();  // 1: chunk totals and the zeroed flag are in place
-    if (rank == 0 && threadIdx.x < 32) {
-      const double tot =
-        summed ? group_chunk_offsets(f, g, threadIdx.x) : 0.0;
-      if (threadIdx.x == 0) {
-        group_finish(f, g, tot, draw);
-      }
+  };
+  if (!active) {
+    move_state();
+    return;
+  }
+  const bool nz = f.gnz[g] != 0;
+  const double mx = ordered_value(f.gkey[g]);
+  const int c0 = f.chunk_first[g];
+  const int nc = f.chunk_count[g];
+  const bool summed = nz && n > 1 && mx != -INFINITY;
+  if (threadIdx.x == 0) {
+    flag = *f.force_serial;
+    s_draw = draw_group_uniform(f, g);  // independent of the weights
+  }
+  if (summed && 32 * (i >> 5) < n) {
+    const bool valid = i < n;
+    const double e = valid ? scaled_weight(f, k, mx) : 0.0;
+    const double incl = warp_inclusive_scan(e);
+    if (valid) {
+      f.ew[k] = e;
+      f.pre[k] = incl;
     }
-    cluster.sync();  // 2: mode, offsets and the target spacing
-    const int mode = f.mode[g];
-    const double uu0 = f.guu0[g];
-    const double du = f.gdu[g];
-    const int c0 = f.chunk_first[g];
-    const int nc = f.chunk_count[g];
-    int* flag0 = cluster.map_shared_rank(&flag, 0);
-    if (mode == MODE_RESAMPLE) {
-      for (int j = threadIdx.x; j < nc; j += TAIL_BLOCK) {
-        s_end[j] = f.chunk_sum[c0 + j];
-        s_off[j] = f.chunk_off[c0 + j];
-      }
-      for (int j = threadIdx.x; j < n; j += TAIL_BLOCK) {
-        s_pre[j] = f.pre[base + j];
-      }
-      __syncthreads();
-      if (i < n) {
-        const search_view sv{s_end, s_off, s_pre, n, nc, uu0, du};
-        const int m = resample_index(sv, i, flag0);
-        f.idx[k] = m;
-        from = base + m;
-      }
-    } else if (mode == MODE_FIRST && i < n) {
-      f.idx[k] = 0;
-      from = base;
-    }
-    cluster.sync();  // 3: every decision and its flag
-    // the same for every block: rank 0's flag is final and no longer
-    // written, the force flag is read-only
-    const bool serial = mode == MODE_RESAMPLE &&
-      (*flag0 != 0 || *f.force_serial != 0);
-    if (serial) {
-      if (rank == 0) {
-        serial_fallback(f, g, count);
-      }
-      cluster.sync();  // 4: the serial indices are in place
-      if (i < n) {
-        from = base + f.idx[k];
-      }
-    } else {
-      // 4, split: rank 0's shared memory must outlive every block's read
-      // of its flag, but the copy below need not wait
-      cluster.barrier_arrive();
-      arrived = true;
+    if ((i & 31) == 31) {
+      f.chunk_sum[c0 + (i >> 5)] = incl;
     }
   }
-  if (i < n) {
-    for (int s = 0; s < n_state; ++s) {
-      dst[static_cast<long>(s) * stride + k] =
-        src[static_cast<long>(s) * stride + from];
+  // 1: chunk totals and prefix sums are in place, and every block has read
+  // the reductions that are cleared below
+  cluster.sync();
+  // one warp scans and draws while the others copy
+  if (threadIdx.x < 32) {
+    double tot = 0;
+    if (summed) {
+      tot = chunk_offsets_warp<MAX / 1024>(f.chunk_sum + c0, nc, s_off,
+                                           s_end);
+    }
+    if (threadIdx.x == 0) {
+      s_total = tot;
+      s_mean = tot / n;
     }
   }
-  if (arrived) {
-    cluster.barrier_wait();
+  if (summed) {
+    const int t = static_cast<int>(threadIdx.x);
+    for (int j = t < 32 ? t + BLOCK - 32 : t - 32; j < n; j += BLOCK) {
+      s_pre[j] = f.pre[base + j];
+    }
   }
+  __syncthreads();
+  const int mode = !nz ? MODE_KEEP : summed ? MODE_RESAMPLE : MODE_FIRST;
+  const double du = s_mean;
+  if (mode == MODE_RESAMPLE) {
+    if (i < n) {
+      const search_view sv{s_end, s_off, s_pre, n, nc, du * s_draw.u, du};
+      int ambiguous = 0;
+      const int m = resample_index(sv, i, &ambiguous);
+      f.idx[k] = m;
+      from = base + m;
+      if (ambiguous) {
+        for (int r = 0; r < TAIL_CLUSTER; ++r) {
+          *cluster.map_shared_rank(&flag, r) = 1;
+        }
+      }
+    }
+  } else if (mode == MODE_FIRST && i < n) {
+    f.idx[k] = 0;
+    from = base;
+  }
+  // the last warp of the last block, which often has the fewest particles
+  const bool records = rank == TAIL_CLUSTER - 1 &&
+    threadIdx.x == BLOCK - 32;
+  double inc = 0;
+  if (records && nz) {
+    inc = n == 1 ? f.w[base] :
+      mode == MODE_FIRST ? -INFINITY : math::log(du) + mx;
+  }
+  move_state();
+  // 2: every decision and its flag; every block has read the generator
+  cluster.sync();
+  if (records) {
+    if (nz) {
+      f.ll[g] += inc;
+      for (int w = 0; w < 4; ++w) {
+        f.frng[8 * g + w] = s_draw.r.state[w];
+      }
+      f.gu[g] = s_draw.u;
+      f.gtot[g] = s_total;
+      f.guu0[g] = du * s_draw.u;
+      f.gdu[g] = du;
+    }
+    f.mode[g] = mode;
+    f.gkey[g] = ordered_key(-INFINITY);
+    f.gnz[g] = 0;
+    f.gflag[g] = 0;
+  }
+  if (mode == MODE_RESAMPLE && flag != 0) {
+    if (rank == 0) {
+      serial_fallback(f, g, s_draw.u, count);
+    }
+    cluster.sync();  // 3: the serial indices are in place
+    if (i < n) {
+      from = base + f.idx[k];
+    }
+    move_state();
+  }
+}
+
+__global__ void __cluster_dims__(TAIL_CLUSTER, 1, 1)
+__launch_bounds__(TAIL_BLOCK)
+k_tail_cluster(filter_view f, int* count, const double* src, double* dst,
+               int stride, int n_state) {
+  tail_cluster<TAIL_BLOCK>(f, count, src, dst, stride, n_state);
+}
+
+__global__ void __cluster_dims__(TAIL_CLUSTER, 1, 1)
+__launch_bounds__(TAIL_BLOCK_LARGE)
+k_tail_cluster_large(filter_view f, int* count, const double* src,
+                     double* dst, int stride, int n_state) {
+  tail_cluster<TAIL_BLOCK_LARGE>(f, count, src, dst, stride, n_state);
 }
 
 // After the reorder of a data time: the saved state entries of each

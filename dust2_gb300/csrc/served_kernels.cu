@@ -66,7 +66,8 @@ __global__ void k_reorder_active(const double* __restrict__ src,
   const int k = tl.start + threadIdx.x;
   const bool move = group_mode[tl.group] != MODE_KEEP;
   const int from = move ? group_offset[tl.group] + index[k] : k;
-  for (int s = 0; s < n_state; ++s) {
+#pragma unroll 4
+  for (int s = blockIdx.y; s < n_state; s += gridDim.y) {
     dst[static_cast<long>(s) * stride + k] =
       src[static_cast<long>(s) * stride + from];
   }
