@@ -516,10 +516,17 @@ public:
         DUST2_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
       }
     }
-    // (a small output is not worth a second launch)
+    // A small output is not worth a second launch, and to pageable memory
+    // one copy is the faster and the steadier way (65,536 ODEs, 29 MB: 8
+    // copies 10.0 to 14.2 ms a run, one 9.8 to 9.9).
+    cudaPointerAttributes where{};
+    const bool pinned =
+      cudaPointerGetAttributes(&where, out) == cudaSuccess &&
+      where.type == cudaMemoryTypeHost;
+    cudaGetLastError();  // an unregistered pointer may be reported as such
     const long n_chunks_worth = static_cast<long>(
       per_time * n_times * sizeof(double) / (1 << 20)) + 1;
-    const int n_chunks = static_cast<int>(std::min<long>(
+    const int n_chunks = !pinned ? 1 : static_cast<int>(std::min<long>(
       std::min(n_times, n_sim_chunks), n_chunks_worth));
     std::vector<int> first(n_chunks + 1);
     for (int c = 0; c <= n_chunks; ++c) {
