@@ -118,8 +118,10 @@ struct state {
   // entries of c4 that interpolate_reset has written since.
   bool pending;
   unsigned c4_set;
-  // log(max(error, 1e-4)), when known
+  // While has_log_error: error is still to be formed as the root of
+  // mean_square, and log_error is 2 log(max(error, 1e-4)).
   bool has_log_error;
+  double mean_square;
   double log_error;
 };
 
@@ -166,6 +168,13 @@ DUST2_HD double div_period(double t, double period) {
   const std::uint64_t b = math::bits_of(period);
   const std::uint64_t e = b >> 52;  // sign and biased exponent
   if ((b & 0x000fffffffffffffull) == 0 && e >= 2 && e <= 2045) {
+    // an exponent subtraction where both are normal
+    const std::uint64_t tb = math::bits_of(t);
+    const std::uint64_t te = (tb >> 52) & 0x7ff;
+    const std::uint64_t qe = te + 1023 - e;
+    if (te - 1 < 2046 && qe - 1 < 2046) {
+      return math::from_bits(tb + ((1023 - e) << 52));
+    }
     return t * math::from_bits((2046 - e) << 52);
   }
   return t / period;
@@ -199,6 +208,15 @@ template <class T>
 struct has_lane_sum<T, std::void_t<decltype(&T::lane_sum)>>
   : std::true_type {};
 
+// A system may say that the rate of entry i is always that of an earlier
+// entry j negated: T::opposite_rate(i) is j, or -1.  Its error estimate is
+// then the other's negated, the same bits.
+template <class T, class = void>
+struct has_opposite_rates : std::false_type {};
+template <class T>
+struct has_opposite_rates<T, std::void_t<decltype(&T::opposite_rate)>>
+  : std::true_type {};
+
 template <typename T, int NV>
 struct solver {
   const control_dev& ctl;
@@ -211,9 +229,14 @@ struct solver {
   int n_special = 0;
   // 1 / n_var for the error norm's mean
   double inv_n_var = 1.0 / n_var;
-  // the controller's constant logarithms
+  // the controller's constants: its logarithms are of the mean square, so
+  // twice those of the error
   double log_safe = math::log(ctl.factor_safe);
-  double log_floor = math::log(1e-4);
+  double log_floor = 2 * math::log(1e-4);
+  double half_constant = 0.5 * ctl.constant;
+  double half_beta = 0.5 * ctl.beta;
+  double inv_facc1 = 1 / ctl.facc1;
+  double inv_facc2 = 1 / ctl.facc2;
 
   // Whether entry i is one of the integrated variables.
   DUST2_HD bool on(int i) const {
@@ -241,21 +264,18 @@ struct solver {
     T::rhs(t, y, shared, internal, dydt);
   }
 
-  // The stages as chains of fused multiply-adds over the tableau's
-  // weights scaled by h once per step: y + h (a_1 k_1 + ... + a_j k_j)
-  // becomes fma(h a_j, k_j, ... fma(h a_1, k_1, y)), j FP64 instructions
-  // per variable instead of 2j + 1.  The rounding differs from the
-  // reference's expression, within the solver's tolerance.
+  // The stages as chains of fused multiply-adds: y + h (a_1 k_1 + ... +
+  // a_j k_j) is j + 1 FP64 instructions per variable, or j with weights
+  // scaled by h once per step, where the stage is short or (the last) of
+  // all variables.  The rounding differs from the reference's expression,
+  // within the solver's tolerance.  Returns the mean square of the scaled
+  // errors.
   DUST2_HD double try_step(double t, double h, const double* y,
                            state<NV>& st, scratch<NV>& s) {
     const double* k1 = st.dydt;
     const double t_next = t + h;
     const double b21 = h * A21;
     const double b31 = h * A31, b32 = h * A32;
-    const double b41 = h * A41, b42 = h * A42, b43 = h * A43;
-    const double b51 = h * A51, b52 = h * A52, b53 = h * A53, b54 = h * A54;
-    const double b61 = h * A61, b62 = h * A62, b63 = h * A63, b64 = h * A64,
-      b65 = h * A65;
     const double b71 = h * A71, b73 = h * A73, b74 = h * A74, b75 = h * A75,
       b76 = h * A76;
 #pragma unroll
@@ -273,30 +293,33 @@ struct solver {
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       if (on(i)) {
-        double acc = std::fma(b41, k1[i], y[i]);
-        acc = std::fma(b42, s.k2[i], acc);
-        s.y_next[i] = std::fma(b43, s.k3[i], acc);
+        double acc = A41 * k1[i];
+        acc = std::fma(A42, s.k2[i], acc);
+        acc = std::fma(A43, s.k3[i], acc);
+        s.y_next[i] = std::fma(h, acc, y[i]);
       }
     }
     rhs(t + C4 * h, s.y_next, s.k4);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       if (on(i)) {
-        double acc = std::fma(b51, k1[i], y[i]);
-        acc = std::fma(b52, s.k2[i], acc);
-        acc = std::fma(b53, s.k3[i], acc);
-        s.y_next[i] = std::fma(b54, s.k4[i], acc);
+        double acc = A51 * k1[i];
+        acc = std::fma(A52, s.k2[i], acc);
+        acc = std::fma(A53, s.k3[i], acc);
+        acc = std::fma(A54, s.k4[i], acc);
+        s.y_next[i] = std::fma(h, acc, y[i]);
       }
     }
     rhs(t + C5 * h, s.y_next, s.k5);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       if (on(i)) {
-        double acc = std::fma(b61, k1[i], y[i]);
-        acc = std::fma(b62, s.k2[i], acc);
-        acc = std::fma(b63, s.k3[i], acc);
-        acc = std::fma(b64, s.k4[i], acc);
-        s.y_stiff[i] = std::fma(b65, s.k5[i], acc);
+        double acc = A61 * k1[i];
+        acc = std::fma(A62, s.k2[i], acc);
+        acc = std::fma(A63, s.k3[i], acc);
+        acc = std::fma(A64, s.k4[i], acc);
+        acc = std::fma(A65, s.k5[i], acc);
+        s.y_stiff[i] = std::fma(h, acc, y[i]);
       }
     }
     rhs(t_next, s.y_stiff, s.k6);
@@ -311,24 +334,29 @@ struct solver {
       }
     }
     rhs(t_next, s.y_next, s.k2);
-    const double e1 = h * E1, e3 = h * E3, e4 = h * E4, e5 = h * E5,
-      e6 = h * E6, e7 = h * E7;
-    double err = 0.0;
+    double err = 0.0;  // of the estimates over h
+    double estimate[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       if (on(i)) {
-        double acc = e1 * k1[i];
-        acc = std::fma(e3, s.k3[i], acc);
-        acc = std::fma(e4, s.k4[i], acc);
-        acc = std::fma(e5, s.k5[i], acc);
-        acc = std::fma(e6, s.k6[i], acc);
-        acc = std::fma(e7, s.k2[i], acc);
+        double acc = E1 * k1[i];
+        acc = std::fma(E3, s.k3[i], acc);
+        acc = std::fma(E4, s.k4[i], acc);
+        acc = std::fma(E5, s.k5[i], acc);
+        acc = std::fma(E6, s.k6[i], acc);
+        acc = std::fma(E7, s.k2[i], acc);
+        if constexpr (has_opposite_rates<T>::value) {
+          // an entry whose rate is that of an earlier one, negated
+          const int j = T::opposite_rate(i);
+          acc = j >= 0 ? -estimate[j >= 0 ? j : 0] : acc;
+        }
+        estimate[i] = acc;
         const double sk = acc *
           recip(std::fma(ctl.rtol, max_abs(y[i], s.y_next[i]), ctl.atol));
         err = std::fma(sk, sk, err);
       }
     }
-    return sqrt(total(err) * inv_n_var);
+    return total(err) * inv_n_var * (h * h);
   }
 
   // The record of an accepted step: what settle and dense_output need and
@@ -361,16 +389,19 @@ struct solver {
     *c3 = std::fma(h, k1, -st.c2[i]);
     *c4 = (st.c4_set >> i) & 1 ? st.c4[i] :
       std::fma(-h, s.k2[i], st.c2[i]) - *c3;
-    double acc = (h * D1) * k1;
-    acc = std::fma(h * D3, s.k3[i], acc);
-    acc = std::fma(h * D4, s.k4[i], acc);
-    acc = std::fma(h * D5, s.k5[i], acc);
-    acc = std::fma(h * D6, s.k6[i], acc);
-    *c5 = std::fma(h * D7, s.k2[i], acc);
+    double acc = D1 * k1;
+    acc = std::fma(D3, s.k3[i], acc);
+    acc = std::fma(D4, s.k4[i], acc);
+    acc = std::fma(D5, s.k5[i], acc);
+    acc = std::fma(D6, s.k6[i], acc);
+    *c5 = h * std::fma(D7, s.k2[i], acc);
   }
 
   // Complete the record, before it is stored.
   DUST2_HD void settle(state<NV>& st, const scratch<NV>& s) const {
+    if (st.has_log_error) {
+      st.error = sqrt(st.mean_square);
+    }
     if (!st.pending) {
       return;
     }
@@ -421,14 +452,15 @@ struct solver {
     if (truncated) {
       h = t_end - t;
     }
-    const double err = try_step(t, h, y, st, s);
+    const double mean_square = try_step(t, h, y, st, s);
     st.n_steps++;
     // The controller's powers through one logarithm and one exponential
     // of the engine (integer fixed point, no FP64 instruction):
-    // err^c / fac_old^beta / safe = exp(c log err - beta log fac_old -
-    // log safe); log 0 = -Inf, and NaN and Inf propagate as through pow.
-    const double log_err = math::log(err);
-    if (err <= 1) {
+    // safe fac_old^beta / err^c = exp(log safe + beta log fac_old -
+    // c log err), the factor of the step size, with the logarithms of
+    // err^2; log 0 = -Inf, and NaN and Inf propagate as through pow.
+    const double log_err = math::log(mean_square);
+    if (mean_square <= 1) {
       update_interpolation(t, h, y, st, s);
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
@@ -442,15 +474,16 @@ struct solver {
       if (!truncated) {
         // log fac_old is the last step's log err, or the floor's
         const double log_old = st.has_log_error ? st.log_error :
-          math::log(ref_max(st.error, 1e-4));
-        const double log_fac = std::fma(ctl.constant, log_err,
-                                        -ctl.beta * log_old) - log_safe;
-        const double fac = clamp(math::exp(log_fac), ctl.facc2, ctl.facc1);
-        const double h_new = h * recip(fac);
+          2 * math::log(ref_max(st.error, 1e-4));
+        const double log_fac = std::fma(-half_constant, log_err,
+                                        half_beta * log_old) + log_safe;
+        const double h_new =
+          h * clamp(math::exp(log_fac), inv_facc1, inv_facc2);
         const double h_max = reject ? h : ctl.step_size_max;
         st.step_size = ref_min(h_new, h_max);
-        st.error = err;
-        st.log_error = err < 1e-4 ? log_floor : log_err;
+        st.mean_square = mean_square;
+        st.log_error = math::gt_nonneg(1e-8, mean_square) ? log_floor :
+          log_err;
         st.has_log_error = true;
       }
       t = truncated ? t_end : t + h;
@@ -460,8 +493,8 @@ struct solver {
     if (st.n_steps_accepted >= 1) {
       st.n_steps_rejected++;
     }
-    h *= recip(ref_min(ctl.facc1, math::exp(std::fma(ctl.constant, log_err,
-                                                     -log_safe))));
+    h *= ref_max(inv_facc1, math::exp(std::fma(-half_constant, log_err,
+                                               log_safe)));
     return 0;
   }
 

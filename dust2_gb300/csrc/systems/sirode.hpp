@@ -18,7 +18,7 @@ struct sirode {
     real_type I0;
     real_type beta;
     real_type gamma;
-    math::divisor by_N;
+    real_type rate;  // beta / N
   };
   struct internal_state {};
   struct data_type {
@@ -42,7 +42,7 @@ struct sirode {
     s.N = read_par<sirode>(pars, 1);
     s.beta = read_par<sirode>(pars, 2);
     s.gamma = read_par<sirode>(pars, 3);
-    s.by_N = math::divisor::of(s.N);
+    s.rate = s.beta / s.N;
     return s;
   }
 
@@ -50,6 +50,12 @@ struct sirode {
     s.I0 = read_par_update<sirode>(pars, 0, s.I0);
     s.beta = read_par_update<sirode>(pars, 2, s.beta);
     s.gamma = read_par_update<sirode>(pars, 3, s.gamma);
+    s.rate = s.beta / s.N;
+  }
+
+  // the rates of cases_cumul and cases_inc are that of S, negated
+  DUST2_HD static constexpr int opposite_rate(int i) {
+    return i >= 3 ? 0 : -1;
   }
 
   static std::vector<packing_entry> packing_state(const shared_state&) {
@@ -88,7 +94,13 @@ struct sirode {
                            real_type* state_deriv) {
     const auto S = state[0];
     const auto I = state[1];
-    const auto rate_SI = math::divide(shared.beta * S * I, shared.by_N);
+#if defined(__CUDA_ARCH__)
+    // 2 FP64 instructions instead of a product and a division (the same
+    // number of roundings)
+    const auto rate_SI = shared.rate * S * I;
+#else
+    const auto rate_SI = shared.beta * S * I / shared.N;
+#endif
     const auto rate_IR = shared.gamma * I;
     state_deriv[0] = -rate_SI;
     state_deriv[1] = rate_SI - rate_IR;
