@@ -569,6 +569,13 @@ DUST2_MATH_CORE double rcp(double y) {
   return std::fma(r, e, r);
 }
 
+// a / b as a call: the rare branch of the functions below.  Written in
+// place, the compiler evaluated the division (some 10 FP64 instructions)
+// whether it was needed or not and selected its result afterwards.
+DUST2_MATH_CORE double divide_call(double a, double b) {
+  return a / b;
+}
+
 // Exact division by a value that is used many times: a / b, correctly
 // rounded, in 4 FP64 instructions instead of an IEEE division's sequence.
 // With hi = RN(1/b) and lo = 1/b - hi, q = fma(a, hi, RN(a lo)) is within
@@ -595,7 +602,7 @@ DUST2_HD double divide_fma(double a, const divisor& d) {
   const int e = static_cast<int>((bits_of(a) >> 52) & 0x7ff);
   if (e < 1023 - 400 || e > 1023 + 400 ||
       (bits_of(d.lo) << 1) > 0xffe0000000000000ull) {
-    return a / d.b;
+    return divide_call(a, d.b);
   }
   const double q = std::fma(a, d.hi, a * d.lo);
   return std::fma(std::fma(-q, d.b, a), d.hi, q);

@@ -177,7 +177,7 @@ DUST2_HD double div_period(double t, double period) {
     }
     return t * math::from_bits((2046 - e) << 52);
   }
-  return t / period;
+  return math::divide_call(t, period);
 }
 
 // 1/x through the engine's reciprocal (an FP32 seed and two Newton steps,
@@ -185,7 +185,7 @@ DUST2_HD double div_period(double t, double period) {
 // elsewhere.  Four FP64 instructions instead of a division's sequence.
 DUST2_HD double recip(double x) {
   const std::uint64_t e = (math::bits_of(x) >> 52) & 0x7ff;
-  return e - (1023 - 99) <= 198 ? math::rcp(x) : 1.0 / x;
+  return e - (1023 - 99) <= 198 ? math::rcp(x) : math::divide_call(1.0, x);
 }
 
 // Systems whose state always has n_state_max entries may declare
@@ -207,6 +207,26 @@ struct has_lane_sum : std::false_type {};
 template <class T>
 struct has_lane_sum<T, std::void_t<decltype(&T::lane_sum)>>
   : std::true_type {};
+
+// The last coefficient of the dense output, and its value at u (v = 1 - u).
+// Called, so that they are evaluated for the entry being reset: expanded
+// under the test of the reset mask they were evaluated ahead of it, for
+// every entry at every step (117 of 293 FP64 instructions of a sirode step
+// between daily outputs, which resets nothing by interpolation).
+DUST2_MATH_CORE double dense_c5(double h, double k1, double k3, double k4,
+                                double k5, double k6, double k7) {
+  double acc = D1 * k1;
+  acc = std::fma(D3, k3, acc);
+  acc = std::fma(D4, k4, acc);
+  acc = std::fma(D5, k5, acc);
+  acc = std::fma(D6, k6, acc);
+  return h * std::fma(D7, k7, acc);
+}
+
+DUST2_MATH_CORE double dense_value(double c1, double c2, double c3, double c4,
+                                   double c5, double u, double v) {
+  return c1 + u * (c2 + v * (c3 + u * (c4 + v * c5)));
+}
 
 // A system may say that the rate of entry i is always that of an earlier
 // entry j negated: T::opposite_rate(i) is j, or -1.  Its error estimate is
@@ -384,17 +404,11 @@ struct solver {
   DUST2_HD void coefficients(int i, const state<NV>& st,
                              const scratch<NV>& s, double* c3, double* c4,
                              double* c5) const {
-    const double h = st.h;
-    const double k1 = st.c3[i];
-    *c3 = std::fma(h, k1, -st.c2[i]);
+    *c3 = std::fma(st.h, st.c3[i], -st.c2[i]);
     *c4 = (st.c4_set >> i) & 1 ? st.c4[i] :
-      std::fma(-h, s.k2[i], st.c2[i]) - *c3;
-    double acc = D1 * k1;
-    acc = std::fma(D3, s.k3[i], acc);
-    acc = std::fma(D4, s.k4[i], acc);
-    acc = std::fma(D5, s.k5[i], acc);
-    acc = std::fma(D6, s.k6[i], acc);
-    *c5 = h * std::fma(D7, s.k2[i], acc);
+      std::fma(-st.h, s.k2[i], st.c2[i]) - *c3;
+    *c5 = dense_c5(st.h, st.c3[i], s.k3[i], s.k4[i], s.k5[i], s.k6[i],
+                   s.k2[i]);
   }
 
   // Complete the record, before it is stored.
@@ -524,8 +538,7 @@ struct solver {
         if (st.pending) {
           coefficients(i, st, s, &c3, &c4, &c5);
         }
-        const double val = st.c1[i] + u * (st.c2[i] + v * (c3 + u *
-                                                           (c4 + v * c5)));
+        const double val = dense_value(st.c1[i], st.c2[i], c3, c4, c5, u, v);
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
           if (q == r) {
