@@ -136,11 +136,10 @@ __device__ __forceinline__ void store_ode_scalars(
 // its state; the rows are shared out over the grid's second dimension.
 template <int NV>
 __global__ void k_reorder_record(ode_view src, ode_view dst,
-                                 const tile* __restrict__ tiles,
-                                 const int* __restrict__ group_offset,
-                                 const int* __restrict__ index,
-                                 const int* __restrict__ group_mode) {
+                                 const tile* tiles, const int* group_offset,
+                                 const int* index, const int* group_mode) {
   const tile tl = tiles[blockIdx.x];
+  previous_done();
   if (static_cast<int>(threadIdx.x) >= tl.count) {
     return;
   }
@@ -720,10 +719,11 @@ public:
   void enqueue_reorder_record(const ode_view& src, const ode_view& dst,
                               const tile* tiles, int n_tiles, int tile_size,
                               const int* group_offset, const int* index,
-                              const int* group_mode, cudaStream_t s) {
-    k_reorder_record<NV><<<dim3(n_tiles, 16), tile_size, 0, s>>>(
-      src, dst, tiles, group_offset, index, group_mode);
-    DUST2_CUDA(cudaGetLastError());
+                              const int* group_mode, bool overlap,
+                              cudaStream_t s) {
+    launch_after_previous(overlap, k_reorder_record<NV>, dim3(n_tiles, 16),
+                          tile_size, 0, s, src, dst, tiles, group_offset,
+                          index, group_mode);
   }
 
 private:

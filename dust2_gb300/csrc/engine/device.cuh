@@ -80,6 +80,39 @@ private:
 
 #if defined(__CUDACC__)
 
+// Programmatic dependent launch.  The kernels of a filter's observation
+// loop follow each other on one stream, each short: launched with
+// launch_after_previous, a kernel's blocks are set up while the one before
+// still runs, and wait in previous_done() until it has finished and its
+// writes are visible.  Every thread of every block calls that before it
+// touches anything the kernels before may write, and before it returns; it
+// then lets the next kernel be set up, so at most one is waiting.  Kernels
+// that call it are free to read run-constant data (tiles, parameters)
+// earlier; their pointers are not __restrict__, which would let the compiler
+// read through them ahead of the wait.  Without the attribute the call does
+// nothing.
+__device__ __forceinline__ void previous_done() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+void launch_after_previous(bool overlap, void (*kernel)(P...), dim3 grid,
+                           dim3 block, std::size_t smem, cudaStream_t s,
+                           A&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  DUST2_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
 __device__ __forceinline__ unsigned long long ordered_key(double d) {
   const unsigned long long u = static_cast<unsigned long long>(
     __double_as_longlong(d));

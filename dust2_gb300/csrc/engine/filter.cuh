@@ -178,6 +178,7 @@ __device__ __forceinline__ void step_compare_tile(
     double time_compare, const typename T::data_type* d) {
   sm.load(v, tl.group);
   sm.load_zero_steps(v, tl.group, time, dt, n_steps);
+  previous_done();
   __syncthreads();
   const bool valid = static_cast<int>(threadIdx.x) < tl.count;
   double logw = 0;
@@ -215,6 +216,7 @@ k_step_compare_mixed(
   constexpr int NV = n_var_max<T>();
   __shared__ shared_smem<T> sm;
   const tile tl = v.tiles[blockIdx.x];
+  previous_done();
   if (!f.active[tl.group]) {
     return;
   }
@@ -284,6 +286,7 @@ __global__ void __launch_bounds__(128) k_step_compare_lanes(
   constexpr int V = lane_system::V;
   constexpr int NV = n_var_max<T>();
   const tile tl = v.tiles[blockIdx.x];
+  previous_done();
   if (!f.active[tl.group]) {
     return;
   }
@@ -400,6 +403,7 @@ DUST2_PARTICLE_KERNEL(T) k_step_compare(system_view<T> v, filter_view f,
   __shared__ shared_smem<T> sm;
   const tile tl = v.tiles[blockIdx.x];
   if (!f.active[tl.group]) {
+    previous_done();
     return;
   }
   step_compare_tile<T>(v, f, tl, sm, time, dt, n_steps, time_compare,
@@ -418,6 +422,7 @@ DUST2_PARTICLE_KERNEL(T) k_step_compare_queue(
     int n_groups_data, int n_tiles, int* next_tile) {
   __shared__ shared_smem<T> sm;
   __shared__ int taken;
+  previous_done();
   for (;;) {
     __syncthreads();  // every warp is done with the last tile's `sm`
     if (threadIdx.x == 0) {
@@ -469,6 +474,8 @@ __device__ __forceinline__ double group_chunk_offsets(const filter_view& f,
 __global__ void k_weights(filter_view f);
 __global__ void k_group(filter_view f, int n_groups);
 __global__ void k_resample(filter_view f);
+// Serial fallback, counting how many groups needed it.
+__global__ void k_fallback_count(filter_view f, int* count);
 // Block size of k_fallback_count (any multiple of 32 up to 1024 works).
 constexpr int FALLBACK_THREADS = 1024;
 // The one-launch tail: a cluster of TAIL_CLUSTER blocks of TAIL_BLOCK
@@ -1117,7 +1124,7 @@ public:
     v.rng = rng;
     v.tiles = step_tiles_.data();
     launch_step_shape(s, f, v, shape_, n_step_tiles_, step_grid_, st, i,
-                      next_tile);
+                      next_tile, !timing_);
   }
 
   // `grid`: the blocks of a persistent launch (persistent_grid, found
@@ -1125,17 +1132,19 @@ public:
   void launch_step_shape(cudaStream_t s, const filter_view& f,
                          const system_view<T>& v, const step_shape& sh,
                          int n_tiles, int grid, const obs_step& st,
-                         std::size_t i, int* next_tile) {
+                         std::size_t i, int* next_tile, bool overlap) {
     auto& S = *sys_;
     const auto* d = data_.data() + i * n_groups_data_;
     const int smem = count_smem_per_thread<T>() * sh.block;
     if (sh.persistent) {
-      k_step_compare_queue<T><<<grid, sh.block, smem, s>>>(
-        v, f, st.t0, S.dt(), st.n_steps, st.t_compare, d, n_groups_data_,
-        n_tiles, next_tile);
+      launch_after_previous(overlap, k_step_compare_queue<T>, grid, sh.block,
+                            smem, s, v, f, st.t0, S.dt(), st.n_steps,
+                            st.t_compare, d, n_groups_data_, n_tiles,
+                            next_tile);
     } else {
-      k_step_compare<T><<<n_tiles, sh.block, smem, s>>>(
-        v, f, st.t0, S.dt(), st.n_steps, st.t_compare, d, n_groups_data_);
+      launch_after_previous(overlap, k_step_compare<T>, n_tiles, sh.block,
+                            smem, s, v, f, st.t0, S.dt(), st.n_steps,
+                            st.t_compare, d, n_groups_data_);
     }
   }
 
@@ -1302,7 +1311,7 @@ public:
         const std::size_t e = 2 * (r * cand.size() + c);
         DUST2_CUDA(cudaEventRecord(ev[e], s));
         launch_step_shape(s, f, w, cand[c], n_tiles[c], grids[c], trial,
-                          mid, counter.data());
+                          mid, counter.data(), false);
         DUST2_CUDA(cudaEventRecord(ev[e + 1], s));
       }
     }
@@ -1403,6 +1412,8 @@ private:
     system_view<T> v = S.view();
     k_initial_flagged<T><<<NT, TS, 0, s>>>(v, set_initial_.data(),
                                            time_start_);
+    // no overlap with events recorded between the launches
+    const bool overlap = !timing_;
     double* cur = S.state_ptr();
     double* other = S.state_other_ptr();
     ode_view record{}, record_other{};
@@ -1420,17 +1431,19 @@ private:
         v.tiles = step_tiles_.data();
         if constexpr (has_lanes<T>::value) {
           if (mixed_lanes_) {
-            k_step_compare_lanes<T><<<n_step_tiles_, 32, 0, s>>>(
-              v, record, owner_->control_dev(), f, st.t0, st.t_compare,
+            launch_after_previous(
+              overlap, k_step_compare_lanes<T>, n_step_tiles_, 32, 0, s, v,
+              record, owner_->control_dev(), f, st.t0, st.t_compare,
               owner_->dt(), i == 0 ? 1 : 0,
               data_.data() + i * n_groups_data_, n_groups_data_);
           }
         }
         if (!mixed_lanes_) {
-          k_step_compare_mixed<T><<<n_step_tiles_, shape_.block, 0, s>>>(
-            v, record, owner_->control_dev(), f, st.t0,
-            st.t_compare, owner_->dt(), i == 0 ? 1 : 0,
-            data_.data() + i * n_groups_data_, n_groups_data_);
+          launch_after_previous(
+            overlap, k_step_compare_mixed<T>, n_step_tiles_, shape_.block, 0,
+            s, v, record, owner_->control_dev(), f, st.t0, st.t_compare,
+            owner_->dt(), i == 0 ? 1 : 0, data_.data() + i * n_groups_data_,
+            n_groups_data_);
         }
       } else {
         launch_step(s, f, v.state, v.rng, st, i, queue_.data() + i);
@@ -1439,22 +1452,26 @@ private:
         this->record(ev_step_[2 * i + 1]);
       }
       if (fused_tail_) {
-        (tail_block_ == TAIL_BLOCK ? k_tail_cluster : k_tail_cluster_large)
-          <<<G * TAIL_CLUSTER, tail_block_, 0, s>>>(
-            f, fallback_count_.data(), cur, other, L.stride,
-            S.n_state() <= TAIL_STATE ? S.n_state() : 0);
+        launch_after_previous(
+          overlap, tail_block_ == TAIL_BLOCK ? k_tail_cluster :
+          k_tail_cluster_large, G * TAIL_CLUSTER, tail_block_, 0, s, f,
+          fallback_count_.data(), cur, other, L.stride,
+          S.n_state() <= TAIL_STATE ? S.n_state() : 0);
       } else {
-        k_weights<<<NT, TS, 0, s>>>(f);
-        k_group<<<G, group_threads_, 0, s>>>(f, G);
-        k_resample<<<NT, TS, 0, s>>>(f);
-        k_fallback_counted(f, s);
+        launch_after_previous(overlap, k_weights, NT, TS, 0, s, f);
+        launch_after_previous(overlap, k_group, G, group_threads_, 0, s, f,
+                              G);
+        launch_after_previous(overlap, k_resample, NT, TS, 0, s, f);
+        launch_after_previous(overlap, k_fallback_count, G, FALLBACK_THREADS,
+                              0, s, f, fallback_count_.data());
       }
       if (!fused_tail_ || S.n_state() > TAIL_STATE) {
         if (timing_ && !fused_tail_) {
           this->record(ev_reorder_[2 * i]);
         }
-        k_reorder<<<reorder_grid(NT, S.n_state()), TS, 0, s>>>(
-          cur, other, L.stride, S.n_state(),
+        launch_after_previous(
+          overlap, k_reorder, reorder_grid(NT, S.n_state()), TS, 0, s, cur,
+          other, L.stride, S.n_state(),
           L.tiles.empty() ? nullptr : S.tiles_dev(), offset_.data(),
           idx_.data(), mode_.data());
         if (timing_ && !fused_tail_) {
@@ -1464,13 +1481,13 @@ private:
       if constexpr (is_continuous<T>()) {
         owner_->enqueue_reorder_record(record, record_other, S.tiles_dev(),
                                        NT, TS, offset_.data(), idx_.data(),
-                                       mode_.data(), s);
+                                       mode_.data(), overlap, s);
         std::swap(record, record_other);
       }
       std::swap(cur, other);
       const std::size_t stride = L.stride;
       if (save_traj_ || !snap_obs_.empty()) {
-        k_save_history<<<NT, TS, 0, s>>>(
+        launch_after_previous(overlap, k_save_history, NT, TS, 0, s,
           cur, L.stride, traj_index_dev_.data(),
           save_traj_ ? n_trajectory_state() : 0, S.tiles_dev(),
           active_.data(), mode_.data(), idx_.data(),
@@ -1479,7 +1496,7 @@ private:
       }
       for (std::size_t sn = 0; sn < snap_obs_.size(); ++sn) {
         if (snap_obs_[sn] == static_cast<int>(i)) {
-          k_save_history<<<NT, TS, 0, s>>>(
+          launch_after_previous(overlap, k_save_history, NT, TS, 0, s,
             cur, L.stride, all_state_dev_.data(), S.n_state(),
             S.tiles_dev(), active_.data(), mode_.data(), idx_.data(),
             snap_state_.data() + sn * S.n_state() * stride, nullptr);
@@ -1494,7 +1511,7 @@ private:
       if constexpr (is_continuous<T>()) {
         owner_->enqueue_reorder_record(record, record_other, S.tiles_dev(),
                                        NT, TS, offset_.data(), nullptr,
-                                       nullptr, s);
+                                       nullptr, false, s);
       }
     }
     if (timing_) {
@@ -1547,8 +1564,6 @@ private:
     run_ms_ += ms;
     n_timed_runs_++;
   }
-
-  void k_fallback_counted(filter_view f, cudaStream_t s);
 
   void capture() {
     auto s = sys_->stream();
@@ -1654,15 +1669,6 @@ private:
   cudaGraphExec_t graph_exec_ = nullptr;
   const double* graph_state_ptr_ = nullptr;
 };
-
-// Serial fallback, counting how many groups needed it.
-__global__ void k_fallback_count(filter_view f, int* count);
-
-template <typename T>
-void filter_engine<T>::k_fallback_counted(filter_view f, cudaStream_t s) {
-  const int G = sys_->layout().n_groups;
-  k_fallback_count<<<G, FALLBACK_THREADS, 0, s>>>(f, fallback_count_.data());
-}
 
 }  // namespace engine
 }  // namespace dust2gpu

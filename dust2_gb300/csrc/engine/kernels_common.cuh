@@ -108,21 +108,32 @@ static __global__ void k_scatter_state(const double* __restrict__ in, int stride
 // dst[s][k] = src[s][offset(group(k)) + index[k]] for every particle of
 // tile blockIdx.x; index is group-local.  Particles of groups whose mode
 // is not "resampled" (mode == nullptr means all are) are copied as is.
-static __global__ void k_reorder(const double* __restrict__ src,
-                          double* __restrict__ dst, int stride, int n_state,
-                          const tile* __restrict__ tiles,
-                          const int* __restrict__ group_offset,
-                          const int* __restrict__ index,
-                          const int* __restrict__ group_mode) {
+static __global__ void k_reorder(const double* src, double* dst, int stride,
+                                 int n_state, const tile* tiles,
+                                 const int* group_offset, const int* index,
+                                 const int* group_mode) {
   const tile tl = tiles[blockIdx.x];
+  previous_done();
   if (static_cast<int>(threadIdx.x) >= tl.count) {
     return;
   }
   const int k = tl.start + threadIdx.x;
   const bool move = group_mode == nullptr || group_mode[tl.group] != 0;
   const int from = move ? group_offset[tl.group] + index[k] : k;
-#pragma unroll 4
-  for (int s = blockIdx.y; s < n_state; s += gridDim.y) {
+  const int step = gridDim.y;
+  int s = blockIdx.y;
+  for (; s + 3 * step < n_state; s += 4 * step) {  // four loads in flight
+    double x[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      x[q] = src[static_cast<long>(s + q * step) * stride + from];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      dst[static_cast<long>(s + q * step) * stride + k] = x[q];
+    }
+  }
+  for (; s < n_state; s += step) {
     dst[static_cast<long>(s) * stride + k] =
       src[static_cast<long>(s) * stride + from];
   }

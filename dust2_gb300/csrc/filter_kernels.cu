@@ -43,6 +43,7 @@ __device__ __forceinline__ double scaled_weight(const filter_view& f, int k,
 
 // exp(w - max), the chunk-local inclusive prefix sums and chunk totals.
 __global__ void k_weights(filter_view f) {
+  previous_done();
   const tile tl = f.tiles[blockIdx.x];
   const int g = tl.group;
   if (!f.active[g] || !f.gnz[g] || f.n_particles[g] == 1) {
@@ -188,6 +189,7 @@ __device__ double group_chunk_offsets_block(const filter_view& f, int g) {
 
 // One block (a multiple of 32 threads, at most 1024) per group.
 __global__ void k_group(filter_view f, int n_groups) {
+  previous_done();
   const int g = blockIdx.x;
   if (g >= n_groups || !f.active[g]) {
     return;
@@ -318,6 +320,7 @@ __device__ int resample_index(const search_view& sv, int i, int* flag) {
 }
 
 __global__ void k_resample(filter_view f) {
+  previous_done();
   const tile tl = f.tiles[blockIdx.x];
   const int g = tl.group;
   if (!f.active[g]) {
@@ -508,6 +511,7 @@ __device__ void serial_fallback(const filter_view& f, int g, double u,
 
 __global__ void __launch_bounds__(FALLBACK_THREADS)
 k_fallback_count(filter_view f, int* count) {
+  previous_done();
   const int g = blockIdx.x;
   if (!f.active[g] || f.mode[g] != MODE_RESAMPLE || !f.gflag[g]) {
     return;
@@ -581,8 +585,8 @@ __device__ __forceinline__ double chunk_offsets_warp(const double* sums,
 // the third exactly when its flag, the same in every block, is set.
 template <int BLOCK>
 __device__ __forceinline__ void tail_cluster(
-    const filter_view& f, int* count, const double* __restrict__ src,
-    double* __restrict__ dst, int stride, int n_state) {
+    const filter_view& f, int* count, const double* src, double* dst,
+    int stride, int n_state) {
   constexpr int MAX = TAIL_CLUSTER * BLOCK;
   __shared__ int flag;  // some decision of the group is ambiguous
   __shared__ double s_end[MAX / 32];
@@ -603,26 +607,37 @@ __device__ __forceinline__ void tail_cluster(
   int from = k;  // the source of this particle's state
   auto move_state = [&] {
     if (i < n) {
-#pragma unroll 8
-      for (int s = 0; s < n_state; ++s) {
-        dst[static_cast<long>(s) * stride + k] =
-          src[static_cast<long>(s) * stride + from];
+      double x[TAIL_STATE];
+#pragma unroll
+      for (int q = 0; q < TAIL_STATE; ++q) {
+        if (q < n_state) {
+          x[q] = src[static_cast<long>(q) * stride + from];
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < TAIL_STATE; ++q) {
+        if (q < n_state) {
+          dst[static_cast<long>(q) * stride + k] = x[q];
+        }
       }
     }
   };
+  const int c0 = f.chunk_first[g];
+  const int nc = f.chunk_count[g];
+  if (threadIdx.x == 0) {
+    flag = *f.force_serial;
+    // independent of the weights, and last written by this kernel for the
+    // data time before, which has finished
+    s_draw = draw_group_uniform(f, g);
+  }
+  previous_done();
   if (!active) {
     move_state();
     return;
   }
   const bool nz = f.gnz[g] != 0;
   const double mx = ordered_value(f.gkey[g]);
-  const int c0 = f.chunk_first[g];
-  const int nc = f.chunk_count[g];
   const bool summed = nz && n > 1 && mx != -INFINITY;
-  if (threadIdx.x == 0) {
-    flag = *f.force_serial;
-    s_draw = draw_group_uniform(f, g);  // independent of the weights
-  }
   if (summed && 32 * (i >> 5) < n) {
     const bool valid = i < n;
     const double e = valid ? scaled_weight(f, k, mx) : 0.0;
@@ -737,6 +752,7 @@ __global__ void k_save_history(const double* state, int stride,
                                const tile* tiles, const int* active,
                                const int* mode, const int* idx,
                                double* hist_state, int* hist_order) {
+  previous_done();
   const tile tl = tiles[blockIdx.x];
   if (!active[tl.group] || static_cast<int>(threadIdx.x) >= tl.count) {
     return;
