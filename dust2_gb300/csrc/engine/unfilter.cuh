@@ -359,10 +359,20 @@ __global__ void __launch_bounds__(128) k_unfilter_adjoint_lanes(
       }
     }
   };
+  // the resets due in the next L steps, each step's test made by one lane
+  std::uint64_t due[ZERO_EVERY_MAX];
   save_step(0);
   for (int step = 0; step < n_steps_total; ++step) {
     const double t = time_start + static_cast<double>(step) * dt;
-    apply_zero_every<T>(zero, nullptr, step, t, x);
+    if (step % L == 0) {
+      const double mine = time_start + static_cast<double>(step + sub) * dt;
+      for (int e = 0; e < zero.n; ++e) {
+        due[e] = __ballot_sync(
+          lanes, math::is_multiple(mine, zero.period[e])) >>
+          (threadIdx.x % 32 / L * L);
+      }
+    }
+    apply_zero_every<T>(zero, due, step % L, t, x);
     double y[NS];
     T::update(t, dt, x, shared, internal, rng, y);
 #pragma unroll

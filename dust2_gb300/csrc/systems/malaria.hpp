@@ -161,8 +161,9 @@ struct malaria {
 #if defined(__CUDACC__)
   // The same equations with a particle's variables shared out over L lanes,
   // V consecutive ones each (the vectors' Ev chain then needs one value of
-  // the lane before).  Every derivative is x y - a s - b s with the terms of
-  // rhs in their order, or x y - a s; entries past the last are 0.
+  // the lane before).  Every derivative is x s - a y - b y with the terms of
+  // rhs in their order, or x s - a y, by fused multiply-adds (one rounding
+  // each where rhs has two); entries past the last are 0.
   template <int L>
   struct lanes {
     using shared_state = malaria::shared_state;
@@ -229,8 +230,8 @@ struct malaria {
         } else if (i >= 4 + in.n) {
           x = 0, s = 0, a = 0, b = 0;
         }
-        const real_type d = x * s - a * y[v];
-        state_deriv[v] = two ? d - b * y[v] : d;
+        const real_type d = std::fma(x, s, -(a * y[v]));
+        state_deriv[v] = two ? std::fma(-b, y[v], d) : d;
       }
     }
 
