@@ -107,14 +107,20 @@ struct shared_smem {
 };
 
 template <typename T>
-__device__ __forceinline__ void load_state(const system_view<T>& v, int k,
-                                           double* x) {
+__device__ __forceinline__ void load_column(const system_view<T>& v,
+                                            const double* from, double* x) {
 #pragma unroll
   for (int s = 0; s < T::n_state_max; ++s) {
     if (s < v.n_state) {
-      x[s] = v.state[static_cast<long>(s) * v.stride + k];
+      x[s] = from[static_cast<long>(s) * v.stride];
     }
   }
+}
+
+template <typename T>
+__device__ __forceinline__ void load_state(const system_view<T>& v, int k,
+                                           double* x) {
+  load_column<T>(v, v.state + k, x);
 }
 
 template <typename T>
@@ -155,6 +161,30 @@ struct state_column {
     return p[s * stride];
   }
 };
+
+// Copy a particle's state, 16 loads in flight.
+template <typename T>
+__device__ __forceinline__ void copy_column(const system_view<T>& v,
+                                            const double* from, double* to) {
+  constexpr int n = T::n_state_max < 16 ? T::n_state_max : 16;
+  const long stride = v.stride;
+#pragma unroll 1
+  for (int s = 0; s < v.n_state; s += n) {
+    double x[n];
+#pragma unroll
+    for (int j = 0; j < n; ++j) {
+      if (s + j < v.n_state) {
+        x[j] = from[(s + j) * stride];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < n; ++j) {
+      if (s + j < v.n_state) {
+        to[(s + j) * stride] = x[j];
+      }
+    }
+  }
+}
 
 // Reset the zero_every entries due at step `step` (time `time`): the
 // first ZERO_STEPS_CACHED steps read the block's precomputed masks.  The
@@ -234,18 +264,19 @@ __device__ __forceinline__ void run_particle(
   }
 }
 
-// Advance particle k n_steps by update() from its state in device memory,
-// and store it again: out of line, for the few particles of a system with
+// Advance particle k n_steps by update() from the state at `from`, and store
+// it: out of line, for the few particles of a system with
 // count_update that cannot be stepped as counts.
 template <typename T>
 __device__ __noinline__ void step_particle_update(
-    const system_view<T>& v, int k, double time, double dt, int n_steps,
-    const typename T::shared_state& shared, const zero_every_spec& z,
-    const std::uint64_t* zero_steps, random::rng_state& rng) {
+    const system_view<T>& v, const double* from, int k, double time,
+    double dt, int n_steps, const typename T::shared_state& shared,
+    const zero_every_spec& z, const std::uint64_t* zero_steps,
+    random::rng_state& rng) {
   typename T::internal_state internal{};
   double x[T::n_state_max];
   double y[update_in_place_of<T>::value ? 1 : T::n_state_max];
-  load_state<T>(v, k, x);
+  load_column<T>(v, from, x);
   run_particle<T>(time, dt, n_steps, shared, internal, z, zero_steps, rng, x,
                   y);
   store_state<T>(v, k, x);
@@ -298,17 +329,19 @@ void allow_count_smem(K kernel) {
   }
 }
 
-// Advance particle k n_steps from its state in device memory and store
-// it again; then done(x, internal) runs on the new state.  Systems with
+// Advance particle k n_steps from the state at `from` (entry s at
+// from[s * stride]: its own, or in a filter its ancestor's in the other
+// buffer) and store it; then done(x, internal) runs on the new state.  Systems with
 // count_update step a particle whose state is counts in FP32
 // (dust2gpu/count_draws.hpp), without an FP64 instruction and with half
 // the registers or local memory; the entries go from memory to FP32 and
 // back by their bits.
 template <typename T, typename F>
 __device__ __forceinline__ void step_particle(
-    const system_view<T>& v, int k, double time, double dt, int n_steps,
-    const typename T::shared_state& shared, const zero_every_spec& z,
-    const std::uint64_t* zero_steps, random::rng_state& rng, const F& done) {
+    const system_view<T>& v, const double* from, int k, double time,
+    double dt, int n_steps, const typename T::shared_state& shared,
+    const zero_every_spec& z, const std::uint64_t* zero_steps,
+    random::rng_state& rng, const F& done) {
   typename T::internal_state internal{};
   double x[T::n_state_max];
   if constexpr (has_count_update<T>::value) {
@@ -316,13 +349,17 @@ __device__ __forceinline__ void step_particle(
     bool ok = !v.deterministic && shared.counts.ready(dt);
     const state_column g{v.state + k, v.stride};
     if constexpr (has_count_layout<T>::value) {
+      if (from != g.p) {
+        copy_column<T>(v, from, g.p);
+      }
       ok = ok && T::count_load(g, c);
     } else if (ok) {
 #pragma unroll
       for (int s = 0; s < T::n_state_max; ++s) {
         float f = 0;
         if (s < v.n_state) {
-          ok &= random::filter::count_of(g[s], &f);
+          ok &= random::filter::count_of(
+            from[static_cast<long>(s) * v.stride], &f);
         }
         c[s] = f;
       }
@@ -355,14 +392,14 @@ __device__ __forceinline__ void step_particle(
       }
     } else {
       random::rng_state r = rng;
-      step_particle_update<T>(v, k, time, dt, n_steps, shared, z, zero_steps,
-                              r);
+      step_particle_update<T>(v, from, k, time, dt, n_steps, shared, z,
+                              zero_steps, r);
       rng = r;
       load_state<T>(v, k, x);
     }
   } else {
     double y[update_in_place_of<T>::value ? 1 : T::n_state_max];
-    load_state<T>(v, k, x);
+    load_column<T>(v, from, x);
     run_particle<T>(time, dt, n_steps, shared, internal, z, zero_steps, rng,
                     x, y);
     store_state<T>(v, k, x);
@@ -463,7 +500,7 @@ DUST2_PARTICLE_KERNEL(T) k_run(system_view<T> v, double time, double dt,
   const auto& shared = mixed ? v.shared[g] : sm.shared();
   const zero_every_spec& zero = mixed ? v.zero_every[g] : sm.zero;
   auto rng = load_rng(v.rng, v.stride, k, v.deterministic);
-  step_particle<T>(v, k, time, dt, n_steps, shared, zero,
+  step_particle<T>(v, v.state + k, k, time, dt, n_steps, shared, zero,
                    mixed ? nullptr : sm.zero_steps, rng,
                    [](const double*, typename T::internal_state&) {});
   store_rng(v.rng, v.stride, k, rng);
@@ -478,6 +515,11 @@ struct run_segment {
 
 // Segments of one k_simulate launch.
 constexpr int MAX_SEGMENTS = 128;
+
+// Doubles of simulate()'s output buffer that a system keeps for its next
+// call (256 MB); a larger one is given back, an allocation being little
+// beside a copy of that size.
+constexpr std::size_t SIM_BUFFER_KEPT = std::size_t(1) << 25;
 
 // Step every particle through `segments`, writing entries index_out (all
 // when null) of its state after each to out[segment][particle][entry].  A
@@ -523,8 +565,8 @@ DUST2_PARTICLE_KERNEL(T) k_simulate(system_view<T> v,
   auto rng = load_rng(v.rng, v.stride, k, v.deterministic);
   for (int i = 0; i < n_segments; ++i) {
     const run_segment seg = segments[i];
-    step_particle<T>(v, k, seg.time, dt, seg.n_steps, shared, zero,
-                     mixed ? nullptr : zero_steps[i], rng,
+    step_particle<T>(v, v.state + k, k, seg.time, dt, seg.n_steps, shared,
+                     zero, mixed ? nullptr : zero_steps[i], rng,
                      [](const double*, typename T::internal_state&) {});
     double* dst = out + (static_cast<long>(i) * n_total + k) * n_out;
     for (int j = 0; j < n_out; ++j) {
@@ -892,6 +934,10 @@ public:
     // as long (96 MB in 8 pieces on a second stream 25 ms, at once 1.2 ms)
     DUST2_CUDA(cudaMemcpyAsync(out, sim_buf_.data(), need * sizeof(double),
                                cudaMemcpyDeviceToHost, stream_));
+    if (need > SIM_BUFFER_KEPT) {
+      sync();
+      sim_buf_.release();
+    }
     check_errors_after();
   }
 

@@ -13,15 +13,16 @@
 //             particle count, data, schedule and generator streams (the
 //             stream layout of a one-group dust2 filter, r/discrete/
 //             filter.hpp:63-75: 2 filter streams then the particles').
-//             Its particle range, generator state and last state stay on
-//             the device between requests.
+//             Its particle range and generator state stay on the device
+//             between requests.
 //   request   one likelihood evaluation of a session at new parameters
 //             (dust_likelihood_run after update_pars): initial state, then
 //             every observation of the session's data.
 //   tick      one observation for every running request: step+compare
 //             (per-session time and data row), weights, log-sum-exp,
-//             resample, reorder: the kernels of the plain filter, over the
-//             tiles of all resident sessions, skipping idle ones.
+//             resample: the kernels of the plain filter, over the
+//             tiles of all resident sessions, skipping idle ones.  A step
+//             reads the particles that the last one's resampling chose.
 //
 // Requests start at the next tick after they arrive, as long as their
 // session is resident and idle; sessions become resident when a slot and
@@ -84,13 +85,6 @@ __global__ void k_served_begin(served_start_list list, filter_view f,
                                int* slot_error);
 __global__ void k_served_advance(int* active, const served_slot* slots,
                                  int* obs, int* starting, int n_slots);
-__global__ void k_reorder_active(const double* __restrict__ src,
-                                 double* __restrict__ dst, int stride,
-                                 int n_state, const tile* __restrict__ tiles,
-                                 const int* __restrict__ active,
-                                 const int* __restrict__ group_offset,
-                                 const int* __restrict__ index,
-                                 const int* __restrict__ group_mode);
 __global__ void k_fallback_count(filter_view f, int* count);
 
 // Initial state of the slots starting a request (filter.hpp:168-172),
@@ -128,6 +122,7 @@ DUST2_PARTICLE_KERNEL(T) k_served_initial(system_view<T> v,
 template <typename T>
 DUST2_PARTICLE_KERNEL(T) k_served_step_compare(system_view<T> v,
                                                filter_view f,
+                                      const double* last_state,
                                       const served_slot* slots,
                                       const int* obs, const obs_step* sched,
                                       const typename T::data_type* data,
@@ -143,7 +138,10 @@ DUST2_PARTICLE_KERNEL(T) k_served_step_compare(system_view<T> v,
   const obs_step st = sched[sl.sched_offset + o];
   system_view<T> vs = v;
   vs.any_error = slot_error + g;
-  step_compare_tile<T>(vs, f, tl, sm, st.t0, sl.dt, st.n_steps,
+  // a request's first step is from the initial state, the others from the
+  // particles that the last observation's resampling chose
+  const step_source src{last_state, o > 0};
+  step_compare_tile<T>(vs, f, tl, sm, src, st.t0, sl.dt, st.n_steps,
                        st.t_compare, data + sl.data_offset + o);
 }
 
@@ -990,8 +988,8 @@ private:
       DUST2_CUDA(cudaEventRecord(r.step0, s));
     }
     k_served_step_compare<T><<<NT, TS, count_smem_per_thread<T>() * TS, s>>>(
-      sview(cur()), f, slots_dev_.data(), obs_dev_.data(), sched_.data(),
-      data_.data(), slot_error_.data());
+      sview(other()), f, cur(), slots_dev_.data(), obs_dev_.data(),
+      sched_.data(), data_.data(), slot_error_.data());
     if (timed) {
       DUST2_CUDA(cudaEventRecord(r.step1, s));
     }
@@ -1000,16 +998,12 @@ private:
     k_resample<<<NT, TS, 0, s>>>(f);
     k_fallback_count<<<S, FALLBACK_THREADS, 0, s>>>(f,
                                                     fallback_count_.data());
-    k_reorder_active<<<reorder_grid(NT, n_state_), TS, 0, s>>>(cur(), other(), cap_particles_,
-                                       n_state_, tiles_.data(),
-                                       active_.data(), offset_.data(),
-                                       idx_.data(), mode_.data());
     k_served_advance<<<n_blocks(S, 128), 128, 0, s>>>(
       active_.data(), slots_dev_.data(), obs_dev_.data(), starting_.data(),
       S);
     DUST2_CUDA(cudaGetLastError());
     parity_ = !parity_;
-    launches_ += 7;
+    launches_ += 6;
     tick_record rec;
     rec.ring = ring_pos_;
     rec.timed = timed;

@@ -1,6 +1,5 @@
 // System-independent kernels of the likelihood server (engine/served.cuh):
-// request start, end-of-tick bookkeeping, and the reorder of running
-// sessions only.
+// request start and end-of-tick bookkeeping.
 #include <cmath>
 
 #include "engine/device.cuh"
@@ -47,29 +46,6 @@ __global__ void k_served_advance(int* active, const served_slot* slots,
   obs[g] = o;
   if (o >= slots[g].n_obs) {
     active[g] = 0;
-  }
-}
-
-// k_reorder (discrete/system.hpp:170-181) restricted to running slots;
-// idle sessions keep their state where it is.
-__global__ void k_reorder_active(const double* __restrict__ src,
-                                 double* __restrict__ dst, int stride,
-                                 int n_state, const tile* __restrict__ tiles,
-                                 const int* __restrict__ active,
-                                 const int* __restrict__ group_offset,
-                                 const int* __restrict__ index,
-                                 const int* __restrict__ group_mode) {
-  const tile tl = tiles[blockIdx.x];
-  if (!active[tl.group] || static_cast<int>(threadIdx.x) >= tl.count) {
-    return;
-  }
-  const int k = tl.start + threadIdx.x;
-  const bool move = group_mode[tl.group] != MODE_KEEP;
-  const int from = move ? group_offset[tl.group] + index[k] : k;
-#pragma unroll 4
-  for (int s = blockIdx.y; s < n_state; s += gridDim.y) {
-    dst[static_cast<long>(s) * stride + k] =
-      src[static_cast<long>(s) * stride + from];
   }
 }
 
