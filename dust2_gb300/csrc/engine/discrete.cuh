@@ -162,27 +162,33 @@ struct state_column {
   }
 };
 
-// Copy a particle's state, 16 loads in flight.
+// Copy a particle's state, 16 loads in flight.  Pointers that move on: with
+// an index per entry the copies were 2.4% of SEIR's step kernel.
 template <typename T>
 __device__ __forceinline__ void copy_column(const system_view<T>& v,
                                             const double* from, double* to) {
   constexpr int n = T::n_state_max < 16 ? T::n_state_max : 16;
   const long stride = v.stride;
+  int s = 0;
 #pragma unroll 1
-  for (int s = 0; s < v.n_state; s += n) {
+  for (; s + n <= v.n_state; s += n) {
     double x[n];
 #pragma unroll
     for (int j = 0; j < n; ++j) {
-      if (s + j < v.n_state) {
-        x[j] = from[(s + j) * stride];
-      }
+      x[j] = *from;
+      from += stride;
     }
 #pragma unroll
     for (int j = 0; j < n; ++j) {
-      if (s + j < v.n_state) {
-        to[(s + j) * stride] = x[j];
-      }
+      *to = x[j];
+      to += stride;
     }
+  }
+#pragma unroll 1
+  for (; s < v.n_state; ++s) {
+    *to = *from;
+    from += stride;
+    to += stride;
   }
 }
 

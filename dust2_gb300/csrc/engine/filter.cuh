@@ -173,11 +173,11 @@ __device__ __forceinline__ void reduce_weight(const filter_view& f, int group,
 // Where a step reads the state of its particles: their own of `state`, or
 // (resampled) those that the resampling chose for them, by f.idx.  `state`
 // is then the other buffer than the one the step writes.  Particles moved so
-// are not read and written once more by k_reorder (58 us an observation of 32
-// x 8192 SEIR particles, 8.4 of 514,064 SIR ones; the step kernels take as
-// long with it as without).  Whole runs, before and after: requests of the
-// likelihood server 52.1 -> 49.4 ms, SEIR 71.0 -> 70.2 ms, batched SIR
-// 33.37 -> 33.08 ms.
+// are not read and written once more by k_reorder: 58 us an observation of
+// 32 x 8192 SEIR particles, for 21 us more in the step kernel (1.09 ms), and
+// 8.4 us of 514,064 SIR particles, for none.  Whole runs, before and after:
+// requests of the likelihood server 52.1 -> 48.8 ms, SEIR 71.0 -> 69.6 ms,
+// batched SIR 33.37 -> 33.05 ms.
 struct step_source {
   const double* state;
   bool resampled;
