@@ -28,12 +28,13 @@ Filter workloads report:
   e2e     the same metric through the public API (dust_likelihood_run:
           parameters copied host->device, log-likelihoods device->host,
           every step), wall-clock;
-  roofline  for the dominant kernel (the step+compare kernel) against the
-          FP64 pipe: executed FP64 operations per particle-step (ncu SASS
-          counters of this kernel, stated in the constant below) times the
-          particle-steps of one launch, over the kernel's device time
-          measured live with CUDA events; peak from a DFMA microbenchmark
-          run in this process; plus the HBM roofline of the reorder gather;
+  roofline  for the dominant kernel (the step+compare kernel): warp
+          instructions per particle-step (ncu, stated in the constants
+          below) times the particle-steps of one launch, over the kernel's
+          device time measured live with CUDA events, against the issue
+          peak; its FP64 work on several bases against a DFMA
+          microbenchmark run in this process; the HBM roofline of the
+          reorder gather;
   cpu_baseline  the CPU restatement of dust2's engine (OpenMP over all
           host cores) on a bounded sample of the same workload.
 
@@ -59,28 +60,33 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
 # Executed FP64 operations (DADD + DMUL + 2 DFMA, per thread) per
-# particle-step of the step+compare kernel, per workload, from the ncu SASS
-# counters of that kernel (summaries under profiles/): whole-run averages
-# of an earlier build, scaled by the ratio of the current build's count to
-# that build's at the same observation (one-launch captures).  A workload
-# without an entry reports no achieved rate.
-FP64_OPS_PER_PARTICLE_STEP = {"sir_batched": 180.9, "seir_batched": 3028.9,
-                              "ode_batched": 552.0}
+# particle-step of the step+compare kernel, or per attempted dopri5 step,
+# from the ncu counters of that kernel (summaries under profiles/): the mean
+# of observations 40, 120 and 200.  A workload without an entry reports no
+# achieved rate.
+FP64_OPS_PER_PARTICLE_STEP = {"sir_batched": 3.5, "seir_batched": 12.4,
+                              "ode_batched": 325.2}
 # FP64-pipe thread instructions (arithmetic, comparisons, conversions) per
 # unit, from the same captures: the pipe's own roofline (every instruction
 # takes one lane-slot; the DFMA peak in TFLOP/s is two flops per slot).
-FP64_PIPE_INST_PER_UNIT = {"sir_batched": 132.7, "seir_batched": 2155.8,
-                           "ode_batched": 351.5}
+FP64_PIPE_INST_PER_UNIT = {"sir_batched": 5.5, "seir_batched": 14.4,
+                           "ode_batched": 217.2}
+# Warp instructions of all kinds per particle-step (smsp__inst_executed.sum
+# of every step launch of a run): the step kernels decide their draws in
+# FP32 and integers, so instruction issue bounds them, one warp instruction
+# per cycle and SM partition.
+WARP_INST_PER_UNIT = {"sir_batched": 36.5, "seir_batched": 605.0}
+PARTITIONS_PER_SM = 4
 
 
 # A second basis for the FP64 roofline, independent of moving work off
 # the FP64 pipe: the FP64 operations (DADD + DMUL + 2 DFMA) the same step
-# kernel executed per particle-step when exp and log were still evaluated
-# in FP64 (Tang's table methods), measured by ncu on that build (whole
-# runs of the batched workloads).  The integer fixed-point exp and log of
-# the current build compute the same values with no FP64 instruction, so
-# this counts the FP64 work of the algorithm as a plain FP64
-# implementation would issue it.
+# kernel executed per particle-step when exp, log and every comparison of
+# the samplers were still evaluated in FP64 (Tang's table methods), measured
+# by ncu on that build (whole runs of the batched workloads).  The current
+# build draws the same values with hardly an FP64 instruction, so this
+# counts the FP64 work of the algorithm as a plain FP64 implementation
+# would issue it, and its fraction may exceed 1.
 FP64_FORMULATION_OPS = {"sir_batched": 259.6, "seir_batched": 4552.2}
 
 
@@ -129,11 +135,10 @@ def algorithmic_roofline(workload, units_per_s, peak_tflops):
 
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per unit of the
-# same kernel, from ncu captures (SIR: a whole run; SEIR: one launch at
-# observation 200, the state in a per-thread local-memory array; dopri5:
-# one launch over all outputs); `traffic` is this times the units of one
+# same kernel, from the same captures (dopri5: one launch over all
+# outputs); `traffic` is this times the units of one
 # launch.
-DRAM_BYTES_PER_UNIT = {"sir_batched": 19.4, "seir_batched": 1598.0,
+DRAM_BYTES_PER_UNIT = {"sir_batched": 26.8, "seir_batched": 798.0,
                        "ode_batched": 36.5}
 
 
@@ -185,6 +190,40 @@ def pipe_roofline(workload, units_per_s, peak_tflops):
     peak = peak_tflops * 1e12 / 2
     return {"inst_per_unit": n, "achieved_inst_per_s": n * units_per_s,
             "peak_inst_per_s": peak, "frac": n * units_per_s / peak}
+
+
+def issue_roofline(workload, kernel, units_per_s, clock_info):
+    """Warp instructions per second of the step kernel against the issue
+    peak (one per cycle and SM partition, at the clock sampled)."""
+    import torch
+    n = WARP_INST_PER_UNIT.get(workload)
+    mhz = clock_info["sm_mhz"]
+    out = {"bound": "issue", "kernel": kernel, "unit": "Gwarp-inst/s",
+           "achieved": None, "peak": None, "frac": None,
+           "peak_source": "SMs x 4 partitions x sampled SM clock"}
+    if n is not None and units_per_s and mhz:
+        sms = torch.cuda.get_device_properties(
+            torch.cuda.current_device()).multi_processor_count
+        out["achieved"] = n * units_per_s / 1e9
+        out["peak"] = sms * PARTITIONS_PER_SM * mhz / 1e3
+        out["frac"] = out["achieved"] / out["peak"]
+        out["warp_inst_per_unit"] = n
+    return out
+
+
+def executed_fp64(workload, units_per_s, peak_tflops):
+    """Executed FP64 operations per second against the DFMA peak."""
+    n = FP64_OPS_PER_PARTICLE_STEP.get(workload)
+    if n is None or not units_per_s:
+        return None
+    return {"flops_per_unit": n, "achieved": n * units_per_s / 1e12,
+            "peak": peak_tflops, "unit": "TFLOP/s",
+            "frac": n * units_per_s / 1e12 / peak_tflops,
+            "peak_source": "measured in-process: DFMA-chain microbenchmark "
+                           "(dust2_gb300_fp64_peak); MEASURED_PEAKS.json "
+                           "has no FP64 entry"}
+
+
 STEPS_PER_OBS = 4  # dt = 0.25, daily observations
 
 
@@ -546,33 +585,21 @@ def gpu_arm(args, rank, world, local):
     if rank == 0:
         peak = fp64_peak_tflops()
         ps_per_launch = n_total * STEPS_PER_OBS
-        achieved = None
-        frac = None
-        ops = FP64_OPS_PER_PARTICLE_STEP.get(args.workload)
-        if ops is not None:
-            achieved = (ops * ps_per_launch / (step_launch_ms * 1e-3) / 1e12)
-            frac = achieved / peak
-        roofline = {
-            "bound": "fp64", "kernel": f"k_step_compare<{w['system']}>",
-            "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-            "frac": frac,
-            "traffic": traffic_per_launch(args.workload, ps_per_launch),
-            "traffic_source": "ncu dram__bytes_read.sum + "
-                              "dram__bytes_write.sum per particle-step of "
-                              "this kernel (DRAM_BYTES_PER_UNIT), times the "
-                              "particle-steps of one launch",
-            "peak_source": "measured in-process: DFMA-chain microbenchmark "
-                           "(dust2_gb300_fp64_peak); MEASURED_PEAKS.json has no FP64 entry",
-            "step_launch_ms": step_launch_ms,
-            "fp64_pipe": pipe_roofline(
-                args.workload, ps_per_launch / (step_launch_ms * 1e-3), peak),
-            "fp64_formulation": formulation_roofline(
-                args.workload, ps_per_launch / (step_launch_ms * 1e-3), peak),
-            "fp64_algorithmic": algorithmic_roofline(
-                args.workload, ps_per_launch / (step_launch_ms * 1e-3), peak),
-            "step_share_of_run": step_ms.value / max(run_ms.value, 1e-12),
-            "flops_basis": "executed FP64 ops per particle-step (ncu SASS "
-                           "dadd+dmul+2*dfma)"}
+        rate = ps_per_launch / (step_launch_ms * 1e-3)
+        roofline = dict(
+            issue_roofline(args.workload, f"k_step_compare<{w['system']}>",
+                           rate, clock_info),
+            traffic=traffic_per_launch(args.workload, ps_per_launch),
+            traffic_source="ncu dram__bytes_read.sum + "
+                           "dram__bytes_write.sum per particle-step of "
+                           "this kernel (DRAM_BYTES_PER_UNIT), times the "
+                           "particle-steps of one launch",
+            step_launch_ms=step_launch_ms,
+            fp64_executed=executed_fp64(args.workload, rate, peak),
+            fp64_pipe=pipe_roofline(args.workload, rate, peak),
+            fp64_formulation=formulation_roofline(args.workload, rate, peak),
+            fp64_algorithmic=algorithmic_roofline(args.workload, rate, peak),
+            step_share_of_run=step_ms.value / max(run_ms.value, 1e-12))
 
     if rank == 0:
         line = {
@@ -588,9 +615,10 @@ def gpu_arm(args, rank, world, local):
                     "d2h_bytes_per_step": d2h, "seconds_per_step": e2e_max},
             # per observation: the step kernel and the tail, which is one
             # cluster launch when every group has <= 1024 particles, else
-            # weights, group, resample, fallback and reorder
+            # weights, group, resample and fallback, and one reorder at
+            # the end of the run
             "gpu_launches": args.steps * (
-                2 + (2 if max(npg) <= 1024 else 6) * n_obs),
+                2 + (2 * n_obs if max(npg) <= 1024 else 5 * n_obs + 1)),
             "clocks": clock_info,
             "roofline": roofline,
             "serial_fallbacks": d.dust_likelihood_serial_fallbacks(obj),
@@ -849,11 +877,8 @@ def serve_arm(args, rank, world, local):
     busy = sum(ps for ps, _ in service) / sum(s for _, s in service)
     weighted = busy / dev["value"]
 
-    ops = FP64_OPS_PER_PARTICLE_STEP.get("seir_batched")
     peak = fp64_peak_tflops()
     in_kernel_rate = total_ps / (step_ms * 1e-3) if step_ms > 0 else None
-    achieved = (ops * in_kernel_rate / 1e12
-                if ops is not None and in_kernel_rate else None)
     n_par = gen.n_pars
     line = {
         "metric": SERVE_METRIC,
@@ -894,27 +919,22 @@ def serve_arm(args, rank, world, local):
                         "log-likelihoods through the server's C ABI"},
         "gpu_launches": launches,
         "clocks": clock_info,
-        "roofline": {
-            "bound": "fp64", "kernel": "k_served_step_compare<seir_age>",
-            "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-            "frac": None if achieved is None else achieved / peak,
-            "traffic": traffic_per_launch(
+        "roofline": dict(
+            issue_roofline("seir_batched", "k_served_step_compare<seir_age>",
+                           in_kernel_rate, clock_info),
+            traffic=traffic_per_launch(
                 "seir_batched",
                 total_ps / max(1, server_info["device_steps"])),
-            "traffic_source": "ncu dram bytes per particle-step of the SEIR "
-                              "step kernel (batched SEIR filter) times the "
-                              "mean particle-steps of one tick",
-            "peak_source": "measured in-process: DFMA-chain microbenchmark "
-                           "(dust2_gb300_fp64_peak); MEASURED_PEAKS.json "
-                           "has no FP64 entry",
-            "step_kernel_share": step_ms * 1e-3 / served_s,
-            "fp64_pipe": pipe_roofline("seir_batched", in_kernel_rate, peak),
-            "fp64_formulation": formulation_roofline("seir_batched",
-                                                     in_kernel_rate, peak),
-            "fp64_algorithmic": algorithmic_roofline("seir_batched",
-                                                     in_kernel_rate, peak),
-            "flops_basis": "executed FP64 ops per particle-step of the "
-                           "SEIR step kernel (ncu SASS dadd+dmul+2*dfma)"},
+            traffic_source="ncu dram bytes per particle-step of the SEIR "
+                           "step kernel (batched SEIR filter) times the "
+                           "mean particle-steps of one tick",
+            step_kernel_share=step_ms * 1e-3 / served_s,
+            fp64_executed=executed_fp64("seir_batched", in_kernel_rate, peak),
+            fp64_pipe=pipe_roofline("seir_batched", in_kernel_rate, peak),
+            fp64_formulation=formulation_roofline("seir_batched",
+                                                  in_kernel_rate, peak),
+            fp64_algorithmic=algorithmic_roofline("seir_batched",
+                                                  in_kernel_rate, peak)),
     }
     if world == 1 and not args.no_cpu_baseline:
         line["cpu_baseline"] = serve_cpu_baseline(w, args.cpu_seconds)

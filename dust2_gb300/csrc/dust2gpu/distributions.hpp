@@ -23,6 +23,11 @@
 // test, so it is evaluated lazily, the first time a candidate falls
 // outside the squeeze; this changes no result.
 //
+// On the device a binomial is decided in FP32 with a bound on every
+// comparison, and evaluated in FP64 as written here only where two sides
+// nearly agree (binomial_filter.hpp): the same integers from the same
+// uniforms.
+//
 // Invalid arguments do not throw (device code cannot): the sampler
 // records the first error in the generator's error slot and returns NaN.
 // Every rejection loop is bounded so that no input can make a kernel spin.

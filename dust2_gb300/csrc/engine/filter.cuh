@@ -46,8 +46,9 @@
 // better than n u relative (u = 2^-53).
 //
 // When every group has at most 1024 particles (4096, for few groups), steps
-// 2-6 run as one launch, k_tail_cluster (a cluster of blocks per group), with the same
-// results.
+// 2-6 run as one launch, k_tail_cluster (a cluster of blocks per group), with
+// the same results.  Each kernel is set up while the one before it runs
+// (programmatic dependent launch) and waits for it before it reads.
 //
 // The whole sequence for all data times is captured once into a CUDA
 // graph and replayed on every run.

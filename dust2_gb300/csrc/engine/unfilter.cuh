@@ -318,7 +318,7 @@ DUST2_PARTICLE_KERNEL(T) k_unfilter_adjoint(
 // those of k_unfilter_adjoint, so the results are the same bits.
 // `n_back[i]`: steps back from data time i to the one before it.  64
 // one-particle groups, 150 daily steps: 1637 us by k_unfilter_adjoint,
-// about 600 us here.
+// 570 us here (a whole gradient call 1.89 -> 0.85 ms).
 template <typename T, int L>
 __global__ void __launch_bounds__(128) k_unfilter_adjoint_lanes(
     system_view<T> v, const int* active, const int* obs_step_index,
