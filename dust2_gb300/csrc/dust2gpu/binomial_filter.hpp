@@ -31,7 +31,7 @@
 // relative elsewhere (the PTX manual's bounds).  The FP64 side's own
 // rounding (at most 5e-7 in the acceptance test, where log k! reaches
 // 2.7e8) is inside the constant terms.  tests/binomial_filter_check.cu
-// measures both sides.
+// compares the draws, with every special-function result moved by its bound.
 #pragma once
 
 #include <cmath>
