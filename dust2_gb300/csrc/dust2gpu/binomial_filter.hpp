@@ -117,7 +117,7 @@ DUST2_HD double count_to_double(float k) {
 }
 
 // A probability in [2^-60, 1/2] as the filter takes it.  `rel` bounds the
-// relative distance of (hi, lo) from the FP64 probability, 0 when they
+// relative distance of all of these from the FP64 probability, 0 when they
 // were made from it.
 struct prob {
   float p;           // 2 e
@@ -142,6 +142,10 @@ DUST2_HD float neg_log1m(float p) {
   s = std::fmaf(s, z2, 1.0f);
   return 2.0f * z * s;
 }
+
+// The largest `rel` that the bounds below have room for; with a larger one
+// (or NaN) every draw is undecided.
+constexpr float REL_MAX = 4 * E;
 
 constexpr std::uint64_t BITS_MIN_P = 0x3c30000000000000ull;  // 2^-60
 
@@ -264,13 +268,14 @@ DUST2_HD float deviance_near(float m, float d) {
 
 // BTRS for n p >= 10.  With c = n p + 1/2 = ci + cf (in integers, cf to
 // 2^-31, n p rel from rel):
-//   g = (2 a / us + b) u and y = cf + g, k = ci + floor(y).  spq has
-//   6 e, b 8 e, a = 0.01 p + 0.0248 b - 0.0873 > 0.08 loses at most a
-//   factor 2.1 and has 22 e.  The uniforms are cut to 32 bits, so us is
-//   also known to 2^-32 only and t = 2 a / us has 27 e + 2^-32 / us; u's
-//   2^-32 adds less than e b.  So y has |u| ((34 e + 2^-32 / us) t +
-//   14 e b), and from cf 2 e: the floor is certain when y is farther than
-//   that from an integer.
+//   g = (2 a / us + b) u and y = cf + g, k = ci + floor(y).  spq, the root
+//   of n p (1 - p), has half of p's own 2 e and of rel (at most 4 e) and of
+//   three roundings, and sqrt's 2 e: 6.5 e; b 8.5 e, and
+//   a = 0.01 p + 0.0248 b - 0.0873 > 0.08 loses at most a factor 2.1 and
+//   has 23 e.  The uniforms are cut to 32 bits, so us is also known to
+//   2^-32 only and t = 2 a / us has 27 e + 2^-32 / us; u's 2^-32 adds less
+//   than e b.  So y has |u| ((34 e + 2^-32 / us) t + 14 e b), and from cf
+//   2 e: the floor is certain when y is farther than that from an integer.
 //   us >= 0.07: certain except for two values of its 32 bits.  v <= v_r,
 //   v_r = 0.92 - 4.2 / b with 4.2 / b < 0.62: 12 e.
 //   The acceptance test's left side log(v alpha / (a / us^2 + b)): 55 e,
@@ -281,10 +286,10 @@ DUST2_HD float deviance_near(float m, float d) {
 //     -[D(k) - D(m)] + 1/2 log(h(m) h(n - m) / (h(k) h(n - k))),
 //     D(x) = deviance(x, n p) + deviance(n - x, n q)
 //   (log x! by h; the linear terms of the two deviances cancel), which
-//   has no large terms: 112 e D(k) + 20 e D(m) + 30 e, 2 |k - n p| rel,
-//   and for the two logarithms of the h (at most 48 in base 2) 4 e of the
-//   first and 120 e.  Where (n + 1) p rounds to the other side of an
-//   integer, f(m) is the same to 2^-24.
+//   has no large terms: 112 e D(k) + 20 e D(m) + 30 e, and for the two
+//   logarithms of the h (at most 48 in base 2) 4 e of the first and 120 e.
+//   From rel, f(k) has 2 |k - n p| rel and f(m) 2 rel; where (n + 1) p
+//   rounds to the other side of an integer, f(m) has 2.1 rel more: 17 e.
 // Returns k, or -1 when undecided (the generator is then at the undecided
 // attempt's first uniform).
 DUST2_HD float btrs(rng_state& rng, float n, const prob& q, float np) {
@@ -359,7 +364,7 @@ DUST2_HD float btrs(rng_state& rng, float n, const prob& q, float np) {
         const float cut = std::fmaf(2.0f, inv_us, rcp32(v));
         const float band = std::fmaf(
           112 * E, d_k, std::fmaf(4 * E, std::fabs(lhs) + std::fabs(lg_h),
-                                  224 * E + cut)) +
+                                  240 * E + cut)) +
           2.0f * q.rel * std::fabs(dk);
         if (diff < -band) {
           return k;
@@ -383,6 +388,9 @@ DUST2_HD float btrs(rng_state& rng, float n, const prob& q, float np) {
 template <typename F>
 DUST2_HD float binomial(rng_state& rng, float n, const prob& q,
                         const F& small) {
+  if (!(q.rel <= REL_MAX)) {
+    return -1.0f;
+  }
   const float np = n * q.p;
   int inv = np < 10.0f ? 1 : 0;
   if (std::fabs(np - 10.0f) <= 10.0f * (8 * E + q.rel)) {
