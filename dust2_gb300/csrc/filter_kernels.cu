@@ -627,14 +627,17 @@ __device__ __forceinline__ void tail_cluster(
   const int nc = f.chunk_count[g];
   if (threadIdx.x == 0) {
     flag = *f.force_serial;
-    // independent of the weights, and last written by this kernel for the
-    // data time before, which has finished
-    s_draw = draw_group_uniform(f, g);
   }
   previous_done();
   if (!active) {
     move_state();
     return;
+  }
+  if (threadIdx.x == 0) {
+    // independent of the weights.  Not before the wait: the generator was
+    // written by this kernel for the data time before, which has finished
+    // by then, but whose writes are only visible after the wait
+    s_draw = draw_group_uniform(f, g);
   }
   const bool nz = f.gnz[g] != 0;
   const double mx = ordered_value(f.gkey[g]);
