@@ -96,7 +96,7 @@ __device__ __forceinline__ void load_ode_scalars(const ode_view& o, int k,
   st.n_steps_rejected = o.n_steps_rejected[k];
   st.err = 0;
   st.pending = false;
-  st.c4_set = 0;
+  st.clear_c4();
   st.has_log_error = false;
   st.log_error = 0;
 }

@@ -118,15 +118,34 @@ struct state {
   // The dense-output record of the last accepted step is formed when it is
   // needed (settle, dense_output).  Until then c1 holds y before the step,
   // c2 its change and c3 the derivative before it; the stages are still in
-  // scratch (k3 .. k6, and the derivative after it in k2).  c4_set marks
-  // entries of c4 that interpolate_reset has written since.
+  // scratch (k3 .. k6, and the derivative after it in k2).  c4_set has a
+  // bit for each entry of c4 that interpolate_reset has written since.
+  static constexpr int c4_words = (NV + 31) / 32;
   bool pending;
-  unsigned c4_set;
+  std::uint32_t c4_set[c4_words];
   // While has_log_error: error is still to be formed as the root of
   // mean_square, and log_error is 2 log(max(error, 1e-4)).
   bool has_log_error;
   double mean_square;
   double log_error;
+
+  DUST2_HD void clear_c4() {
+#pragma unroll
+    for (int w = 0; w < c4_words; ++w) {
+      c4_set[w] = 0;
+    }
+  }
+  DUST2_HD void mark_c4(int i) {
+#pragma unroll
+    for (int w = 0; w < c4_words; ++w) {
+      if (w == i / 32) {
+        c4_set[w] |= 1u << (i % 32);
+      }
+    }
+  }
+  DUST2_HD bool c4_marked(int i) const {
+    return (c4_set[i / 32] >> (i % 32)) & 1;
+  }
 };
 
 template <int NV>
@@ -393,7 +412,7 @@ struct solver {
     st.t1 = t + h;
     st.h = h;
     st.pending = true;
-    st.c4_set = 0;
+    st.clear_c4();
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       if (on(i)) {
@@ -409,7 +428,7 @@ struct solver {
                              const scratch<NV>& s, double* c3, double* c4,
                              double* c5) const {
     *c3 = std::fma(st.h, st.c3[i], -st.c2[i]);
-    *c4 = (st.c4_set >> i) & 1 ? st.c4[i] :
+    *c4 = st.c4_marked(i) ? st.c4[i] :
       std::fma(-st.h, s.k2[i], st.c2[i]) - *c3;
     *c5 = dense_c5(st.h, st.c3[i], s.k3[i], s.k4[i], s.k5[i], s.k6[i],
                    s.k2[i]);
@@ -549,7 +568,7 @@ struct solver {
             st.c4[q] = val;
           }
         }
-        st.c4_set |= 1u << r;
+        st.mark_c4(r);
         ++r;
       }
     }

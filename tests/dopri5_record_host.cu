@@ -1,0 +1,107 @@
+// The engine's dopri5 solver (engine/dopri5.cuh) compiled for the host, for
+// tests of what it keeps between steps: the dense-output record, and resets
+// that are interpolated from it.
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+
+#include "engine/dopri5.cuh"
+
+namespace {
+
+namespace dp = dust2gpu::engine::dopri5;
+using dust2gpu::zero_every_spec;
+
+// `copies` times the same four variables, the last two reset every time
+// unit.
+template <int COPIES>
+struct copies {
+  static constexpr int n = 4 * COPIES;
+  struct shared_state {};
+  struct internal_state {};
+
+  static void rhs(double t, const double* y, const shared_state&,
+                  internal_state&, double* d) {
+    for (int c = 0; c < n; c += 4) {
+      const double s = std::sin(1.3 * t);
+      d[c] = 0.4 * y[c] * (1 - y[c] / 10) + 0.2 * s;
+      d[c + 1] = 0.3 * y[c] - 0.2 * y[c + 1];
+      d[c + 2] = 0.3 * y[c];
+      d[c + 3] = 2 + s;
+    }
+  }
+  static void start(double* y) {
+    for (int c = 0; c < n; c += 4) {
+      y[c] = 1;
+      y[c + 1] = y[c + 2] = y[c + 3] = 0;
+    }
+  }
+  static zero_every_spec zero_every() {
+    std::vector<int> index;
+    for (int c = 0; c < n; c += 4) {
+      index.push_back(c + 2);
+      index.push_back(c + 3);
+    }
+    auto z = dust2gpu::zero_every_none();
+    dust2gpu::zero_every_add(z, 1, index);
+    return z;
+  }
+};
+
+dp::control_dev control(double tol) {
+  dp::control_dev c{};
+  c.max_steps = 10000;
+  c.atol = c.rtol = tol;
+  c.step_size_min = 2.3e-16;
+  c.step_size_max = 1e300;
+  c.factor_safe = 0.9;
+  c.facc1 = 1 / 0.2;
+  c.facc2 = 1 / 10.0;
+  c.beta = 0.04;
+  c.constant = 0.2 - 0.04 * 0.75;
+  return c;
+}
+
+template <int COPIES>
+int wide(const double* times, int n_times, double tol, double* out,
+         double* c4) {
+  using T = copies<COPIES>;
+  constexpr int NV = T::n;
+  const auto c = control(tol);
+  const typename T::shared_state sh{};
+  typename T::internal_state internal{};
+  const auto z = T::zero_every();
+  double y[NV];
+  T::start(y);
+  dp::state<NV> st{};
+  dp::scratch<NV> s{};
+  dp::solver<T, NV> sol{c, sh, internal, NV, 0};
+  sol.initialise(0.0, y, st, s);
+  st.step_size = 0.01;  // initialise()'s depends on the number of variables
+  double t = 0;
+  for (int i = 0; i < n_times; ++i) {
+    sol.run(t, times[i], y, z, st, s);
+    t = times[i];
+    std::memcpy(out + static_cast<long>(i) * NV, y, sizeof(y));
+  }
+  sol.settle(st, s);
+  std::memcpy(c4, st.c4, sizeof(st.c4));
+  return st.err;
+}
+
+}  // namespace
+
+// Integrate `n_copies` copies (1, 8 or 10) of the four variables through
+// `times`: the state at each, and the record's c4 at the end.
+extern "C" int host_copies(int n_copies, const double* times, int n_times,
+                           double tol, double* out, double* c4) {
+  switch (n_copies) {
+  case 1:
+    return wide<1>(times, n_times, tol, out, c4);
+  case 8:
+    return wide<8>(times, n_times, tol, out, c4);
+  case 10:
+    return wide<10>(times, n_times, tol, out, c4);
+  }
+  return -1;
+}

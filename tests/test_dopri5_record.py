@@ -1,0 +1,60 @@
+"""What the engine's dopri5 solver keeps between steps: its own code
+(dust2_gb300/csrc/engine/dopri5.cuh) compiled for the host."""
+import ctypes
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+
+
+def dptr(a):
+    return a.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not shutil.which(nvcc):
+        pytest.skip("nvcc not available")
+    lib = tmp_path_factory.mktemp("record") / "libdopri5_record.so"
+    subprocess.run(
+        [nvcc, "-std=c++17", "-O2", "-shared", "-Xcompiler",
+         "-fPIC,-ffp-contract=off", "-I", str(ROOT / "dust2_gb300" / "csrc"),
+         "-gencode", "arch=compute_103a,code=sm_103a",
+         str(ROOT / "tests" / "dopri5_record_host.cu"), "-o", str(lib)],
+        check=True, capture_output=True)
+    return ctypes.CDLL(str(lib))
+
+
+def copies(host, n_copies, times, tol=1e-6):
+    times = np.asarray(times, dtype=float)
+    out = np.empty((times.size, n_copies, 4))
+    c4 = np.empty((n_copies, 4))
+    rc = host.host_copies(n_copies, dptr(times), times.size,
+                          ctypes.c_double(tol), dptr(out), dptr(c4))
+    assert rc == 0
+    return out, c4
+
+
+@pytest.mark.parametrize("n_copies", [8, 10])
+def test_resets_of_many_variables(host, n_copies):
+    """Copies of four variables, two of them reset by interpolation: 32
+    variables, and 40 (a reset mask of more than one word).  The error norm
+    is a mean over variables and the first step is given, so the copies take
+    the single system's steps up to rounding; 1e-9 is far above what 30 steps of rounding amount to
+    and far below a reset's size (about 1)."""
+    times = [0.7, 1.9, 3.35, 5.45, 9.8]
+    one, one_c4 = copies(host, 1, times)
+    many, many_c4 = copies(host, n_copies, times)
+    np.testing.assert_allclose(many, np.broadcast_to(one, many.shape),
+                               rtol=1e-9, atol=1e-9)
+    # the record: a reset leaves its values in the first entries of c4, two
+    # per copy; the others are the coefficients
+    first = 2 * n_copies
+    np.testing.assert_allclose(
+        many_c4.ravel()[first:],
+        np.broadcast_to(one_c4, many_c4.shape).ravel()[first:],
+        rtol=1e-6, atol=1e-9)
