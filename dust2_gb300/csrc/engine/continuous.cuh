@@ -50,7 +50,7 @@ struct ode_view {
   double* t1;
   double* h;
   double* step_size;
-  double* error;
+  double* mean_square;
   int* n_steps;
   int* n_steps_accepted;
   int* n_steps_rejected;
@@ -90,7 +90,7 @@ __device__ __forceinline__ void load_ode_scalars(const ode_view& o, int k,
   st.t1 = o.t1[k];
   st.h = o.h[k];
   st.step_size = o.step_size[k];
-  st.error = o.error[k];
+  st.mean_square = o.mean_square[k];
   st.n_steps = o.n_steps[k];
   st.n_steps_accepted = o.n_steps_accepted[k];
   st.n_steps_rejected = o.n_steps_rejected[k];
@@ -126,7 +126,7 @@ __device__ __forceinline__ void store_ode_scalars(
   o.t1[k] = st.t1;
   o.h[k] = st.h;
   o.step_size[k] = st.step_size;
-  o.error[k] = st.error;
+  o.mean_square[k] = st.mean_square;
   o.n_steps[k] = st.n_steps;
   o.n_steps_accepted[k] = st.n_steps_accepted;
   o.n_steps_rejected[k] = st.n_steps_rejected;
@@ -159,7 +159,7 @@ __global__ void k_reorder_record(ode_view src, ode_view dst,
     dst.t1[k] = src.t1[from];
     dst.h[k] = src.h[from];
     dst.step_size[k] = src.step_size[from];
-    dst.error[k] = src.error[from];
+    dst.mean_square[k] = src.mean_square[from];
     dst.n_steps[k] = src.n_steps[from];
     dst.n_steps_accepted[k] = src.n_steps_accepted[from];
     dst.n_steps_rejected[k] = src.n_steps_rejected[from];
@@ -355,7 +355,7 @@ public:
     t1_.resize(S);
     h_.resize(S);
     step_size_.resize(S);
-    error_.resize(S);
+    mean_square_.resize(S);
     n_steps_.resize(S);
     n_acc_.resize(S);
     n_rej_.resize(S);
@@ -596,7 +596,7 @@ public:
     move(t1_.data(), 1);
     move(h_.data(), 1);
     move(step_size_.data(), 1);
-    move(error_.data(), 1);
+    move(mean_square_.data(), 1);
     DUST2_CUDA(cudaGetLastError());
     base_.sync();
     // integer counters: reorder on the host (small)
@@ -627,12 +627,12 @@ public:
   std::vector<ode_internals_row> ode_internals() override {
     const auto& L = base_.layout();
     const int N = L.n_total;
-    std::vector<double> ss(N), er(N);
+    std::vector<double> ss(N), ms(N);
     std::vector<int> ns(N), na(N), nr(N);
     DUST2_CUDA(cudaMemcpy(ss.data(), step_size_.data(), N * sizeof(double),
                           cudaMemcpyDeviceToHost));
-    DUST2_CUDA(cudaMemcpy(er.data(), error_.data(), N * sizeof(double),
-                          cudaMemcpyDeviceToHost));
+    DUST2_CUDA(cudaMemcpy(ms.data(), mean_square_.data(),
+                          N * sizeof(double), cudaMemcpyDeviceToHost));
     DUST2_CUDA(cudaMemcpy(ns.data(), n_steps_.data(), N * sizeof(int),
                           cudaMemcpyDeviceToHost));
     DUST2_CUDA(cudaMemcpy(na.data(), n_acc_.data(), N * sizeof(int),
@@ -641,7 +641,8 @@ public:
                           cudaMemcpyDeviceToHost));
     std::vector<ode_internals_row> ret(N);
     for (int k = 0; k < N; ++k) {
-      ret[k] = ode_internals_row{ss[k], er[k], ns[k], na[k], nr[k]};
+      ret[k] = ode_internals_row{ss[k], std::sqrt(ms[k]), ns[k], na[k],
+                                 nr[k]};
     }
     return ret;
   }
@@ -697,7 +698,7 @@ public:
 
   ode_view view_ode() {
     return ode_view{dydt_.data(), c_.data(), t0_.data(), t1_.data(),
-                    h_.data(), step_size_.data(), error_.data(),
+                    h_.data(), step_size_.data(), mean_square_.data(),
                     n_steps_.data(), n_acc_.data(), n_rej_.data(),
                     base_.layout().stride};
   }
@@ -816,7 +817,7 @@ private:
     z(t1_);
     z(h_);
     z(step_size_);
-    z(error_);
+    z(mean_square_);
     z(n_steps_);
     z(n_acc_);
     z(n_rej_);
@@ -828,7 +829,7 @@ private:
   ode_control control_;
   double dt_ = 0;
   std::vector<int> requires_initialise_;
-  device_array<double> dydt_, c_, t0_, t1_, h_, step_size_, error_;
+  device_array<double> dydt_, c_, t0_, t1_, h_, step_size_, mean_square_;
   device_array<int> n_steps_, n_acc_, n_rej_;
   device_array<double> critical_;
   device_array<double> step_times_;

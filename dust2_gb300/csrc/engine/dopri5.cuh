@@ -110,7 +110,7 @@ struct state {
   double t1;
   double h;          // last.h
   double step_size;
-  double error;
+  double mean_square;  // dust2's error, squared
   int n_steps;
   int n_steps_accepted;
   int n_steps_rejected;
@@ -123,10 +123,9 @@ struct state {
   static constexpr int c4_words = (NV + 31) / 32;
   bool pending;
   std::uint32_t c4_set[c4_words];
-  // While has_log_error: error is still to be formed as the root of
-  // mean_square, and log_error is 2 log(max(error, 1e-4)).
+  // While has_log_error, log_error is that of mean_square (below 1e-8,
+  // log_floor).
   bool has_log_error;
-  double mean_square;
   double log_error;
 
   DUST2_HD void clear_c4() {
@@ -286,6 +285,11 @@ struct solver {
     return has_fixed_n_state<T>::value || i < n_var;
   }
 
+  // log(max(mean_square, 1e-8)), given log_ms = log(mean_square)
+  DUST2_HD double floored_log(double mean_square, double log_ms) const {
+    return math::gt_nonneg(1e-8, mean_square) ? log_floor : log_ms;
+  }
+
   DUST2_HD double total(double x) const {
     if constexpr (has_lane_sum<T>::value) {
       return T::lane_sum(internal, x);
@@ -436,9 +440,6 @@ struct solver {
 
   // Complete the record, before it is stored.
   DUST2_HD void settle(state<NV>& st, const scratch<NV>& s) const {
-    if (st.has_log_error) {
-      st.error = sqrt(st.mean_square);
-    }
     if (!st.pending) {
       return;
     }
@@ -511,7 +512,7 @@ struct solver {
       if (!truncated) {
         // log fac_old is the last step's log err, or the floor's
         const double log_old = st.has_log_error ? st.log_error :
-          2 * math::log(ref_max(st.error, 1e-4));
+          floored_log(st.mean_square, math::log(st.mean_square));
         const double log_fac = std::fma(-half_constant, log_err,
                                         half_beta * log_old) + log_safe;
         const double h_new =
@@ -519,8 +520,7 @@ struct solver {
         const double h_max = reject ? h : ctl.step_size_max;
         st.step_size = ref_min(h_new, h_max);
         st.mean_square = mean_square;
-        st.log_error = math::gt_nonneg(1e-8, mean_square) ? log_floor :
-          log_err;
+        st.log_error = floored_log(mean_square, log_err);
         st.has_log_error = true;
       }
       t = truncated ? t_end : t + h;
@@ -672,7 +672,7 @@ struct solver {
   DUST2_HD void initialise(double t, const double* y, state<NV>& st,
                            scratch<NV>& s) {
     st.step_size = 0;
-    st.error = 0;
+    st.mean_square = 0;
     st.has_log_error = false;
     st.n_steps = 0;
     st.n_steps_accepted = 0;

@@ -6,6 +6,7 @@
 #include <cstring>
 
 #include "engine/dopri5.cuh"
+#include "systems/sirode.hpp"
 
 namespace {
 
@@ -104,4 +105,43 @@ extern "C" int host_copies(int n_copies, const double* times, int n_times,
     return wide<10>(times, n_times, tol, out, c4);
   }
   return -1;
+}
+
+// A sirode instance integrated to `times` in one go, or (parts) with its
+// solver record stored and loaded after each of them: the state at the end,
+// the next step size and the squared error.
+extern "C" int host_sirode(const double* pars, const double* times,
+                           int n_times, int parts, double* out) {
+  using T = dust2gpu::systems::sirode;
+  constexpr int NV = 5;
+  const auto c = control(1e-6);
+  const auto sh = T::build_shared(pars);
+  const auto z = T::zero_every(sh);
+  typename T::internal_state internal{};
+  dust2gpu::random::rng_state r{};
+  double y[NV];
+  T::initial(0.0, sh, internal, r, y);
+  dp::state<NV> st{};
+  dp::scratch<NV> s{};
+  dp::solver<T, NV> sol{c, sh, internal, NV, 0};
+  sol.initialise(0.0, y, st, s);
+  double t = 0;
+  for (int i = 0; i < n_times; ++i) {
+    sol.run(t, times[i], y, z, st, s);
+    t = times[i];
+    if (parts) {
+      sol.settle(st, s);
+      // as load_ode leaves what is not stored
+      st.pending = false;
+      st.clear_c4();
+      st.has_log_error = false;
+      st.log_error = 0;
+      s = dp::scratch<NV>{};
+    }
+  }
+  sol.settle(st, s);
+  std::memcpy(out, y, sizeof(y));
+  out[5] = st.step_size;
+  std::memcpy(out + 6, st.c4, sizeof(st.c4));
+  return st.err;
 }

@@ -58,3 +58,40 @@ def test_resets_of_many_variables(host, n_copies):
         many_c4.ravel()[first:],
         np.broadcast_to(one_c4, many_c4.shape).ravel()[first:],
         rtol=1e-6, atol=1e-9)
+
+
+@pytest.mark.parametrize("every", [1.0, 3.3])
+def test_integration_in_parts(host, every):
+    """One run over several output times, and a run to each with the solver
+    record stored in between (dust_system_run_to_time, or output copied in
+    parts): the same bits."""
+    times = every * np.arange(1.0, 31)
+    for k in range(200):
+        pars = np.array([10.0 + k, 1000 + 13.0 * k, 0.2 + 0.002 * k, 0.1])
+        got = np.empty((2, 11))
+        for parts in range(2):
+            assert host.host_sirode(dptr(pars), dptr(times), times.size,
+                                    parts, dptr(got[parts])) == 0
+        np.testing.assert_array_equal(got[0], got[1])
+
+
+@pytest.mark.gpu
+def test_simulate_equals_runs_on_device(built):
+    """As above through the public verbs, and the reported errors."""
+    import dust2_gb300 as d
+    pars = [{"I0": 10.0 + k, "N": 1000 + 13.0 * k, "beta": 0.2 + 0.002 * k,
+             "gamma": 0.1} for k in range(200)]
+    times = 3.3 * np.arange(1.0, 21)
+    whole = d.dust_system_create(d.sirode(), pars, n_groups=200)
+    d.dust_system_set_state_initial(whole)
+    want = d.dust_system_simulate(whole, times)
+    parts = d.dust_system_create(d.sirode(), pars, n_groups=200)
+    d.dust_system_set_state_initial(parts)
+    for i, t in enumerate(times):
+        d.dust_system_run_to_time(parts, t)
+        np.testing.assert_array_equal(d.dust_system_state(parts),
+                                      want[..., i])
+    a, b = d.dust_system_internals(whole), d.dust_system_internals(parts)
+    for name in ("step_size", "error", "n_steps", "n_steps_rejected"):
+        np.testing.assert_array_equal(a[name], b[name])
+    assert np.all(a["error"] > 0) and np.all(a["error"] <= 1)
