@@ -116,7 +116,7 @@ struct state {
   int n_steps_rejected;
   int err;           // error code (0 = none)
   // The dense-output record of the last accepted step is formed when it is
-  // needed (settle, dense_output).  Until then c1 holds y before the step,
+  // needed (settle, interpolate_reset).  Until then c1 holds y before the step,
   // c2 its change and c3 the derivative before it; the stages are still in
   // scratch (k3 .. k6, and the derivative after it in k2).  c4_set has a
   // bit for each entry of c4 that interpolate_reset has written since.
@@ -427,13 +427,23 @@ struct solver {
     }
   }
 
+  // Coefficients 3 and 4 of entry i of a pending record; `after` is the
+  // derivative after its step.
+  DUST2_HD double coefficient3(int i, const state<NV>& st) const {
+    return std::fma(st.h, st.c3[i], -st.c2[i]);
+  }
+  DUST2_HD double coefficient4(int i, const state<NV>& st, double c3,
+                               double after) const {
+    return st.c4_marked(i) ? st.c4[i] :
+      std::fma(-st.h, after, st.c2[i]) - c3;
+  }
+
   // Coefficients 3 to 5 of entry i of a pending record.
   DUST2_HD void coefficients(int i, const state<NV>& st,
                              const scratch<NV>& s, double* c3, double* c4,
                              double* c5) const {
-    *c3 = std::fma(st.h, st.c3[i], -st.c2[i]);
-    *c4 = st.c4_marked(i) ? st.c4[i] :
-      std::fma(-st.h, s.k2[i], st.c2[i]) - *c3;
+    *c3 = coefficient3(i, st);
+    *c4 = coefficient4(i, st, *c3, s.k2[i]);
     *c5 = dense_c5(st.h, st.c3[i], s.k3[i], s.k4[i], s.k5[i], s.k6[i],
                    s.k2[i]);
   }
@@ -456,6 +466,29 @@ struct solver {
     st.pending = false;
   }
 
+  // The record when the solver gives up after a rejected step: that step
+  // has overwritten the stages.  The accepted step's coefficients are
+  // completed (the derivative after it is st.dydt), and c5 is the rejected
+  // step's, as the reference forms it in every trial step (solver.hpp
+  // try_step); st.t1 holds that step's size.
+  DUST2_HD void keep_after_rejection(state<NV>& st,
+                                     const scratch<NV>& s) const {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      if (on(i)) {
+        if (st.pending) {
+          const double c3 = coefficient3(i, st);
+          st.c4[i] = coefficient4(i, st, c3, st.dydt[i]);
+          st.c3[i] = c3;
+        }
+        st.c5[i] = dense_c5(st.t1, st.dydt[i], s.k3[i], s.k4[i], s.k5[i],
+                            s.k6[i], s.k2[i]);
+      }
+    }
+    st.t1 = st.t0 + st.h;
+    st.pending = false;
+  }
+
   DUST2_HD void record_step_time(double t) {
     if (ctl.step_times != nullptr) {
       int& n = ctl.n_step_times[particle];
@@ -474,16 +507,14 @@ struct solver {
   // error (st.err set, t unchanged).
   DUST2_HD int attempt(double& t, double t_end, double* y, double& h,
                        bool& reject, state<NV>& st, scratch<NV>& s) {
-    if (st.n_steps > ctl.max_steps) {
-      st.err = ERR_ODE_TOO_MANY_STEPS;
-      return -1;
-    }
-    if (h < ctl.step_size_min) {
-      st.err = ERR_ODE_STEP_TOO_SMALL;
-      return -1;
-    }
-    if (h <= fabs(t) * 2.220446049250313e-16) {
-      st.err = ERR_ODE_STEP_VANISHED;
+    const int err = st.n_steps > ctl.max_steps ? ERR_ODE_TOO_MANY_STEPS :
+      h < ctl.step_size_min ? ERR_ODE_STEP_TOO_SMALL :
+      h <= fabs(t) * 2.220446049250313e-16 ? ERR_ODE_STEP_VANISHED : 0;
+    if (err != 0) {
+      st.err = err;
+      if (reject) {
+        keep_after_rejection(st, s);
+      }
       return -1;
     }
     const bool truncated = t + h > t_end;
@@ -527,6 +558,7 @@ struct solver {
       return 1;
     }
     reject = true;
+    st.t1 = h;  // until the next accepted step, or keep_after_rejection
     if (st.n_steps_accepted >= 1) {
       st.n_steps_rejected++;
     }
@@ -681,6 +713,17 @@ struct solver {
       ctl.n_step_times[particle] = 0;
     }
     record_step_time(t);
+    if (st.pending) {
+      // c4 needs the derivative after the record's step, which may be
+      // wanted once the stages are gone (keep_after_rejection)
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        if (on(i)) {
+          st.c4[i] = coefficient4(i, st, coefficient3(i, st), s.k2[i]);
+          st.mark_c4(i);
+        }
+      }
+    }
     double* f0 = st.dydt;
     double* f1 = s.y_stiff;  // not the stages of a pending record
     double* y1 = s.y_next;

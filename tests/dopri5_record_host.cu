@@ -145,3 +145,79 @@ extern "C" int host_sirode(const double* pars, const double* times,
   std::memcpy(out + 6, st.c4, sizeof(st.c4));
   return st.err;
 }
+
+namespace {
+
+// Rejected steps at the kick, and more after it.
+struct kicked {
+  struct shared_state {};
+  struct internal_state {};
+  static void rhs(double t, const double* y, const shared_state&,
+                  internal_state&, double* d) {
+    d[0] = t < 5 ? 0.1 * y[0] : -200 * std::sin(40 * t) * y[0];
+    d[1] = y[0] - 0.3 * y[1];
+  }
+};
+
+}  // namespace
+
+// Integrate until the solver gives up (max_steps, or ssmin), one attempt at
+// a time.  got: t0, t1, h and c1 .. c5 as settled afterwards; want: those of
+// the last accepted step, taken when it was made, with c5 of the last
+// attempt.  Returns the error, or -1 without one by time 12; *n_rejected
+// counts the attempts rejected at the end.
+extern "C" int host_give_up(int max_steps, double ssmin, double* got,
+                            double* want, int* n_rejected) {
+  constexpr int NV = 2;
+  auto c = control(1e-6);
+  c.max_steps = max_steps;
+  c.step_size_min = ssmin;
+  const kicked::shared_state sh{};
+  kicked::internal_state internal{};
+  double y[NV] = {1, 0};
+  dp::state<NV> st{};
+  dp::scratch<NV> s{};
+  dp::solver<kicked, NV> sol{c, sh, internal, NV, 0};
+  sol.initialise(0.0, y, st, s);
+  auto put = [](const dp::state<NV>& x, double* out) {
+    out[0] = x.t0;
+    out[1] = x.t1;
+    out[2] = x.h;
+    for (int i = 0; i < NV; ++i) {
+      out[3 + i] = x.c1[i];
+      out[5 + i] = x.c2[i];
+      out[7 + i] = x.c3[i];
+      out[9 + i] = x.c4[i];
+      out[11 + i] = x.c5[i];
+    }
+  };
+  put(st, want);
+  const double end = 12;
+  double t = 0;
+  while (t < end) {
+    bool reject = false;
+    double h = st.step_size;
+    *n_rejected = 0;
+    for (;;) {
+      const double trial = t + h > end ? end - t : h;
+      const int res = sol.attempt(t, end, y, h, reject, st, s);
+      if (res < 0) {
+        sol.settle(st, s);
+        put(st, got);
+        return st.err;
+      }
+      if (res > 0) {
+        auto settled = st;
+        sol.settle(settled, s);
+        put(settled, want);
+        break;
+      }
+      ++*n_rejected;
+      for (int i = 0; i < NV; ++i) {
+        want[11 + i] = dp::dense_c5(trial, st.dydt[i], s.k3[i], s.k4[i],
+                                    s.k5[i], s.k6[i], s.k2[i]);
+      }
+    }
+  }
+  return -1;
+}

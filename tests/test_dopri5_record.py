@@ -75,6 +75,24 @@ def test_integration_in_parts(host, every):
         np.testing.assert_array_equal(got[0], got[1])
 
 
+def test_record_when_the_solver_gives_up(host):
+    """The dense-output record after an error, with and without rejected
+    steps before it."""
+    seen = set()
+    for max_steps, ssmin in ([(n, 2.3e-16) for n in range(0, 120)] +
+                             [(10000, 10.0 ** -k) for k in range(1, 5)]):
+        got, want = np.zeros(13), np.zeros(13)
+        n_rejected = ctypes.c_int()
+        err = host.host_give_up(max_steps, ctypes.c_double(ssmin), dptr(got),
+                                dptr(want), ctypes.byref(n_rejected))
+        if err == -1:
+            continue
+        assert err > 0
+        seen.add((err, min(n_rejected.value, 2)))
+        np.testing.assert_array_equal(got, want)
+    assert len(seen) >= 4  # both errors; no, one and several rejections
+
+
 @pytest.mark.gpu
 def test_simulate_equals_runs_on_device(built):
     """As above through the public verbs, and the reported errors."""
