@@ -223,7 +223,8 @@ struct has_fixed_n_state<T, std::void_t<decltype(T::fixed_n_state)>>
 
 // A system whose variables are shared out over lanes (each integrates its
 // own) sums the error norms over them: T::lane_sum(internal, x), the same
-// value in every lane.
+// value in every lane.  T::holds(internal, i) says whether a lane's entry i
+// is a variable; the others pad it, with value and rate 0.
 template <class T, class = void>
 struct has_lane_sum : std::false_type {};
 template <class T>
@@ -288,6 +289,17 @@ struct solver {
   // log(max(mean_square, 1e-8)), given log_ms = log(mean_square)
   DUST2_HD double floored_log(double mean_square, double log_ms) const {
     return math::gt_nonneg(1e-8, mean_square) ? log_floor : log_ms;
+  }
+
+  // The inverse of the scale of entry i's errors; 0 for padding, which has
+  // no scale when atol is 0.
+  DUST2_HD double inv_scale(int i, double abs_y) const {
+    const double r = recip(std::fma(ctl.rtol, abs_y, ctl.atol));
+    if constexpr (has_lane_sum<T>::value) {
+      return T::holds(internal, i) ? r : 0.0;
+    } else {
+      return r;
+    }
   }
 
   DUST2_HD double total(double x) const {
@@ -398,8 +410,7 @@ struct solver {
           acc = j >= 0 ? -estimate[j >= 0 ? j : 0] : acc;
         }
         estimate[i] = acc;
-        const double sk = acc *
-          recip(std::fma(ctl.rtol, max_abs(y[i], s.y_next[i]), ctl.atol));
+        const double sk = acc * inv_scale(i, max_abs(y[i], s.y_next[i]));
         err = std::fma(sk, sk, err);
       }
     }
@@ -737,7 +748,7 @@ struct solver {
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       if (on(i)) {
-        inv_sk[i] = recip(std::fma(ctl.rtol, fabs(y[i]), ctl.atol));
+        inv_sk[i] = inv_scale(i, fabs(y[i]));
         const double f = f0[i] * inv_sk[i];
         const double g = y[i] * inv_sk[i];
         norm_f = std::fma(f, f, norm_f);

@@ -182,6 +182,10 @@ struct malaria {
       return __shfl_sync(in.mask, y[I % V], I / V, L);
     }
 
+    __device__ static bool holds(const internal_state& in, int v) {
+      return in.lane * V + v < 4 + in.n;
+    }
+
     __device__ static real_type lane_sum(const internal_state& in,
                                          real_type x) {
 #pragma unroll
