@@ -678,10 +678,7 @@ public:
     DUST2_CUDA(cudaMemsetAsync(state_other_.data(), 0,
                                state_other_.size() * sizeof(double), stream_));
     upload_shared();
-    std::vector<zero_every_spec> z;
-    for (auto& s : shared_) {
-      z.push_back(T::zero_every(s));
-    }
+    const std::vector<zero_every_spec> z = zero_every_specs();
     DUST2_CUDA(cudaMemcpyAsync(zero_dev_.data(), z.data(),
                                z.size() * sizeof(zero_every_spec),
                                cudaMemcpyHostToDevice, stream_));
@@ -1035,6 +1032,15 @@ public:
 
   void sync() {
     DUST2_CUDA(cudaStreamSynchronize(stream_));
+  }
+
+  // The groups' resets.
+  std::vector<zero_every_spec> zero_every_specs() const {
+    std::vector<zero_every_spec> z;
+    for (auto& sh : shared_) {
+      z.push_back(T::zero_every(sh));
+    }
+    return z;
   }
 
   void upload_shared() {

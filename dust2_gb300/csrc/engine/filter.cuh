@@ -290,14 +290,28 @@ k_step_compare_mixed(
 }
 
 // Mixed-time systems that can share a particle's variables out over lanes
-// (T::lanes<L>, a system for dopri5::solver that integrates V variables per
-// lane).
+// declare T::lanes<L>, a system for dopri5::solver that integrates V
+// consecutive variables per lane, with
+//   holds(in, v), lane_sum(in, x): see dopri5.cuh;
+//   start(lane, mask, n_var, special): the internal_state of a lane; `mask`
+//     has the particle's lanes of the warp, n_var the particle's variables,
+//     `special` the value of its special entry;
+//   special(in): that entry, by reference;
+//   update_special(time, dt, in, shared, rng): what update() makes of it
+//     (the variables stay as they are).
+// They have one special entry and no outputs, and are used where no group
+// has resets (no_resets); others are integrated by a thread per particle.
 constexpr int MIXED_LANES = 8;
 template <class T, class = void>
 struct has_lanes : std::false_type {};
 template <class T>
 struct has_lanes<T, std::void_t<typename T::template lanes<MIXED_LANES>>>
-  : std::true_type {};
+  : std::integral_constant<bool, n_special<T>() == 1 && T::n_output == 0> {};
+
+inline bool no_resets(const std::vector<zero_every_spec>& groups) {
+  return std::all_of(groups.begin(), groups.end(),
+                     [](const zero_every_spec& z) { return z.n == 0; });
+}
 
 // k_step_compare_mixed with MIXED_LANES lanes per particle, four particles
 // to a warp, for few particles: the stage sums of a lane are those of V
@@ -330,11 +344,8 @@ __global__ void __launch_bounds__(128) k_step_compare_lanes(
     const auto rng = load_rng(v.rng, v.stride, k, v.deterministic);
     const int n_var = v.n_state - T::n_output - n_special<T>();
     const long S = v.stride;
-    typename lane_system::internal_state in;
-    in.lane = sub;
-    in.mask = ((1u << L) - 1u) << (threadIdx.x % 32 / L * L);
-    in.n = n_var - 4;
-    in.beta = v.state[n_var * S + k];
+    const unsigned mask = ((1u << L) - 1u) << (threadIdx.x % 32 / L * L);
+    auto in = lane_system::start(sub, mask, n_var, v.state[n_var * S + k]);
     double y[V];
     dopri5::state<V> st;
     dopri5::scratch<V> s;
@@ -371,19 +382,19 @@ __global__ void __launch_bounds__(128) k_step_compare_lanes(
           break;
         }
         random::rng_state r = rng;
-        const double beta = lane_system::update_special(dt, in.beta, shared,
-                                                        r);
+        const double special = lane_system::update_special(time, dt, in,
+                                                           shared, r);
         if (r.err != 0) {
           update_err = r.err;
           break;
         }
-        bool changed = !(beta == in.beta);
+        bool changed = !(special == lane_system::special(in));
 #pragma unroll
         for (int q = 0; q < V; ++q) {
           changed = changed || y[q] != y[q];
         }
-        in.beta = beta;
-        if (__any_sync(in.mask, changed)) {
+        lane_system::special(in) = special;
+        if (__any_sync(mask, changed)) {
           sol.initialise(time0, y, st, s);
         }
       }
@@ -402,9 +413,9 @@ __global__ void __launch_bounds__(128) k_step_compare_lanes(
         o.c[(4 * NV + i) * S + k] = st.c5[q];
       }
     }
-    __syncwarp(in.mask);
+    __syncwarp(mask);
     if (sub == 0) {
-      v.state[n_var * S + k] = in.beta;
+      v.state[n_var * S + k] = lane_system::special(in);
       store_ode_scalars(o, k, st);
       double x[T::n_state_max];
       load_state<T>(v, k, x);  // what the comparison reads of it
@@ -416,7 +427,6 @@ __global__ void __launch_bounds__(128) k_step_compare_lanes(
         r.err = st.err != 0 ? st.err : update_err;
       }
       capture_error(v.errors, v.any_error, k, r);
-      store_rng(v.rng, v.stride, k, r);
       f.w[k] = logw;
     }
   }
@@ -643,7 +653,7 @@ public:
       // a warp of up to 32.
       constexpr int per_warp = 32 / MIXED_LANES;
       mixed_lanes_ = has_lanes<T>::value && owner_->dt() > 0 &&
-        N <= 3 * per_warp * 4 * n_sms();
+        no_resets(sys_->zero_every_specs()) && N <= 3 * per_warp * 4 * n_sms();
       if (mixed_lanes_) {
         first = step_shape{32, per_warp, false};
       }

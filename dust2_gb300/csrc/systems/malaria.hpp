@@ -176,6 +176,15 @@ struct malaria {
     static constexpr int V = (4 + n_rates_max + L - 1) / L;
     static constexpr bool fixed_n_state = true;
 
+    __device__ static internal_state start(int lane, unsigned mask, int n_var,
+                                           real_type special) {
+      return internal_state{lane, mask, n_var - 4, special};
+    }
+
+    __device__ static real_type& special(internal_state& in) {
+      return in.beta;
+    }
+
     template <int I>
     __device__ static real_type get(const internal_state& in,
                                     const real_type* y) {
@@ -241,9 +250,9 @@ struct malaria {
 
     // update() on the special entry alone.
     __device__ static real_type update_special(
-        real_type dt, real_type beta, const shared_state& shared,
-        rng_state_type& rng_state) {
-      return beta * math::exp(
+        real_type time, real_type dt, const internal_state& in,
+        const shared_state& shared, rng_state_type& rng_state) {
+      return in.beta * math::exp(
         random::normal(rng_state, 0, shared.beta_volatility));
     }
   };
