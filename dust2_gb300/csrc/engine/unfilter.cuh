@@ -421,6 +421,15 @@ __global__ void __launch_bounds__(128) k_unfilter_adjoint_lanes(
     for (int q = 0; q < m; ++q) {
       acc += __shfl_sync(lanes, value, q, L);
     }
+    // an error of the earliest of these data times, whichever lane had it
+    const unsigned failed = __ballot_sync(lanes, rng.err != 0) >>
+      (threadIdx.x % 32 / L * L);
+    if (failed != 0) {
+      const int first = __ffs(static_cast<int>(failed)) - 1;
+      rng.err = __shfl_sync(lanes, rng.err, first, L);
+      rng.err_v0 = __shfl_sync(lanes, rng.err_v0, first, L);
+      rng.err_v1 = __shfl_sync(lanes, rng.err_v1, first, L);
+    }
   }
   double adj[NA];
   double adj_next[NA];
