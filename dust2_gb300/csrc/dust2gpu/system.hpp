@@ -269,16 +269,6 @@ void prepare_counts(typename T::shared_state& shared, double dt) {
   }
 }
 
-// Bytes of those tables.
-template <typename T>
-constexpr std::size_t count_table_bytes() {
-  if constexpr (has_count_update<T>::value) {
-    return sizeof(T::shared_state::counts);
-  } else {
-    return 0;
-  }
-}
-
 // Mixed time: an ODE (rhs) with a discrete-time update applied every dt
 // (properties.hpp:99 is_mixed_time, continuous/system.hpp:544-585).
 template <typename T>

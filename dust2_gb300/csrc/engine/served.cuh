@@ -293,15 +293,14 @@ public:
       throw std::runtime_error("The HBM budget must be positive");
     }
     DUST2_CUDA(cudaGetDevice(&device_));
-    // memory plan: 1/16 of the budget for data and schedules, the rest
-    // for particles (the slots' count tables, about 1 KB each, come on
-    // top)
+    // memory plan: 1/16 of the budget for data and schedules, the slots'
+    // parameters (with their count tables) and bookkeeping, the rest for
+    // particles
     const double per_obs = sizeof(data_type) + sizeof(obs_step);
     long n_obs_cap = static_cast<long>(hbm_budget_bytes / 16 / per_obs);
     n_obs_cap = std::max(1024L, std::min(n_obs_cap, 1L << 26));
     const double slot_bytes = static_cast<double>(n_slots_) *
-      (sizeof(shared_state) - count_table_bytes<T>() +
-       sizeof(zero_every_spec) + 256);
+      (sizeof(shared_state) + sizeof(zero_every_spec) + 256);
     double left = hbm_budget_bytes - n_obs_cap * per_obs - slot_bytes;
     long n_cap = static_cast<long>(left / bytes_per_particle());
     n_cap = std::min(n_cap, 1L << 29) / ALIGN * ALIGN;
