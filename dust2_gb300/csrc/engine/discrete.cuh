@@ -454,6 +454,22 @@ struct min_blocks_of<T, std::void_t<decltype(T::min_blocks_per_sm)>> {
   __global__ void __launch_bounds__(default_tile_size<T>(),               \
                                     min_blocks_of<T>::value)
 
+// The same for the kernels that step particles as counts (step_particle),
+// which need fewer registers than update() in FP64: a system may declare
+// `step_blocks_per_sm` for them.  The deterministic likelihood's kernels run
+// update(), and lose by such a cap: 4096 SEIR particles, 60 data times,
+// 33.7 ms at 4 blocks per SM, 39.2 at 5.
+template <typename T, typename = void>
+struct step_blocks_of : min_blocks_of<T> {};
+template <typename T>
+struct step_blocks_of<T, std::void_t<decltype(T::step_blocks_per_sm)>> {
+  static constexpr int value = T::step_blocks_per_sm;
+};
+
+#define DUST2_STEP_KERNEL(T)                                              \
+  __global__ void __launch_bounds__(default_tile_size<T>(),               \
+                                    step_blocks_of<T>::value)
+
 // The per-particle kernels below run over a layout's run tiles: a block
 // whose particles share one group stages that group's shared state in
 // shared memory; in a packed tile each thread reads its own group's from
@@ -488,8 +504,8 @@ DUST2_PARTICLE_KERNEL(T) k_initial(system_view<T> v, const int* active,
 }
 
 template <typename T>
-DUST2_PARTICLE_KERNEL(T) k_run(system_view<T> v, double time, double dt,
-                               int n_steps) {
+DUST2_STEP_KERNEL(T) k_run(system_view<T> v, double time, double dt,
+                           int n_steps) {
   __shared__ shared_smem<T> sm;
   const tile tl = v.tiles[blockIdx.x];
   const bool mixed = tl.group < 0;
@@ -533,11 +549,11 @@ constexpr std::size_t SIM_BUFFER_KEPT = std::size_t(1) << 25;
 // waiting for the slowest warp each time: 100,003 SIR particles, 60 days of
 // 4 steps, 2.8 ms in 120 launches.
 template <typename T>
-DUST2_PARTICLE_KERNEL(T) k_simulate(system_view<T> v,
-                                    const run_segment* segments,
-                                    int n_segments, double dt, int n_total,
-                                    const int* index_out, int n_out,
-                                    double* out) {
+DUST2_STEP_KERNEL(T) k_simulate(system_view<T> v,
+                                const run_segment* segments,
+                                int n_segments, double dt, int n_total,
+                                const int* index_out, int n_out,
+                                double* out) {
   __shared__ shared_smem<T> sm;
   __shared__ std::uint64_t zero_steps[MAX_SEGMENTS][ZERO_EVERY_MAX];
   const tile tl = v.tiles[blockIdx.x];

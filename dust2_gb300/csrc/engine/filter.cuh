@@ -435,11 +435,11 @@ __global__ void __launch_bounds__(128) k_step_compare_lanes(
 }
 
 template <typename T>
-DUST2_PARTICLE_KERNEL(T) k_step_compare(system_view<T> v, filter_view f,
-                                        step_source src, double time,
-                               double dt, int n_steps, double time_compare,
-                               const typename T::data_type* data,
-                               int n_groups_data) {
+DUST2_STEP_KERNEL(T) k_step_compare(system_view<T> v, filter_view f,
+                                    step_source src, double time, double dt,
+                                    int n_steps, double time_compare,
+                                    const typename T::data_type* data,
+                                    int n_groups_data) {
   __shared__ shared_smem<T> sm;
   const tile tl = v.tiles[blockIdx.x];
   if (!f.active[tl.group]) {
@@ -457,7 +457,7 @@ DUST2_PARTICLE_KERNEL(T) k_step_compare(system_view<T> v, filter_view f,
 // groups of very different sizes then share one launch without a block
 // per tile, and a block that finishes early takes the next tile at once.
 template <typename T>
-DUST2_PARTICLE_KERNEL(T) k_step_compare_queue(
+DUST2_STEP_KERNEL(T) k_step_compare_queue(
     system_view<T> v, filter_view f, step_source src, double time, double dt,
     int n_steps, double time_compare, const typename T::data_type* data,
     int n_groups_data, int n_tiles, int* next_tile) {

@@ -28,7 +28,12 @@ struct seir_age {
   // 4 blocks 77.1 ms, 5 72.5, 6 92.5 (the L1 cache that is left no longer
   // holds what 80 registers spill).  All 96 entries as FP32 in local
   // memory (L1 hit rate 49%) 84.0 ms, in shared memory 88.5.
-  static constexpr int min_blocks_per_sm = 5;
+  static constexpr int step_blocks_per_sm = 5;
+  // Stepped by update(), the 96 doubles are a thread's own array in local
+  // memory: 4 blocks of 128 threads, 128 registers.  Deterministic
+  // likelihood of 4096 particles, 60 data times of 4 steps: 33.7 ms; 5
+  // blocks 39.2.
+  static constexpr int min_blocks_per_sm = 4;
   using real_type = double;
   using rng_state_type = random::rng_state;
   static constexpr int n_age = 16;

@@ -29,7 +29,7 @@ struct sir {
 
   // 64 registers: 32 warps per SM.  The batched SIR filter, ms per run: 2
   // blocks per SM 41.3, 3 39.4, 4 39.0.
-  static constexpr int min_blocks_per_sm = 4;
+  static constexpr int step_blocks_per_sm = 4;
   static constexpr int n_state_max = 5;
   static constexpr real_type default_dt = 1;
   // state entries and the gradient of beta, gamma, I0 (sir.cpp:122-124)

@@ -42,7 +42,7 @@ struct sir_cases {
 
   // 64 registers: 32 warps per SM.  The batched SIR filter, ms per run: 2
   // blocks per SM 41.3, 3 39.4, 4 39.0.
-  static constexpr int min_blocks_per_sm = 4;
+  static constexpr int step_blocks_per_sm = 4;
   static constexpr int n_state_max = 4;
   static constexpr real_type default_dt = 0.25;
 

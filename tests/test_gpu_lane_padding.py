@@ -17,7 +17,7 @@ def final_state(n_particles, n_rates, initial):
     data = {"time": times, "tested": np.array([50.0, np.nan, 80, 20]),
             "positive": np.full(4, np.nan)}
     control = dict(d.dust_ode_control(), atol=0.0)
-    obj = d.dust_filter_create(d.malaria(), 0, data, dt=0.5, seed=4,
+    obj = d.dust_filter_create(d.malaria(), 0, data, dt=1, seed=4,
                                n_particles=n_particles, ode_control=control)
     d.dust_likelihood_run(obj, {"n_rates": n_rates, "a": 0.3},
                           initial=np.repeat(initial[:, None], n_particles,
