@@ -535,8 +535,16 @@ struct run_segment {
   int n_steps;
 };
 
-// Segments of one k_simulate launch.
+// Segments of one k_simulate launch, and their cached reset tests (as
+// load_zero_steps; [segment][entry of the zero_every table]).  A system
+// whose parameters leave no room for these in a block's 48 KB of static
+// shared memory makes the tests particle by particle.
 constexpr int MAX_SEGMENTS = 128;
+using segment_steps = std::uint64_t[MAX_SEGMENTS][ZERO_EVERY_MAX];
+template <typename T>
+constexpr bool segment_steps_fit() {
+  return sizeof(shared_smem<T>) + sizeof(segment_steps) <= 48 * 1024;
+}
 
 // Doubles of simulate()'s output buffer that a system keeps for its next
 // call (256 MB); a larger one is given back, an allocation being little
@@ -555,12 +563,14 @@ DUST2_STEP_KERNEL(T) k_simulate(system_view<T> v,
                                 const int* index_out, int n_out,
                                 double* out) {
   __shared__ shared_smem<T> sm;
-  __shared__ std::uint64_t zero_steps[MAX_SEGMENTS][ZERO_EVERY_MAX];
+  __shared__ std::conditional_t<segment_steps_fit<T>(), segment_steps,
+                                std::uint64_t[1][1]> zero_steps;
   const tile tl = v.tiles[blockIdx.x];
   const bool mixed = tl.group < 0;
   if (!mixed) {
     sm.load(v, tl.group);
-    // the zero_every tests of each segment's first steps, as load_zero_steps
+  }
+  if (segment_steps_fit<T>() && !mixed) {
     const zero_every_spec& z = v.zero_every[tl.group];
     for (int i = threadIdx.x; i < n_segments; i += blockDim.x) {
       const run_segment seg = segments[i];
@@ -588,7 +598,8 @@ DUST2_STEP_KERNEL(T) k_simulate(system_view<T> v,
   for (int i = 0; i < n_segments; ++i) {
     const run_segment seg = segments[i];
     step_particle<T>(v, v.state + k, k, seg.time, dt, seg.n_steps, shared,
-                     zero, mixed ? nullptr : zero_steps[i], rng,
+                     zero, segment_steps_fit<T>() && !mixed ?
+                     zero_steps[i] : nullptr, rng,
                      [](const double*, typename T::internal_state&) {});
     double* dst = out + (static_cast<long>(i) * n_total + k) * n_out;
     for (int j = 0; j < n_out; ++j) {
