@@ -337,12 +337,12 @@ void allow_count_smem(K kernel) {
 
 // Advance particle k n_steps from the state at `from` (entry s at
 // from[s * stride]: its own, or in a filter its ancestor's in the other
-// buffer) and store it; then done(x, internal) runs on the new state.  Systems with
-// count_update step a particle whose state is counts in FP32
-// (dust2gpu/count_draws.hpp), without an FP64 instruction and with half
-// the registers or local memory; the entries go from memory to FP32 and
-// back by their bits.
-template <typename T, typename F>
+// buffer) and store it; then done(x, internal) runs on the new state.  With
+// COUNTS (systems with count_update), a particle whose state is counts is
+// stepped in FP32 (dust2gpu/count_draws.hpp), without an FP64 instruction
+// and with half the registers or local memory; the entries go from memory to
+// FP32 and back by their bits.
+template <typename T, bool COUNTS, typename F>
 __device__ __forceinline__ void step_particle(
     const system_view<T>& v, const double* from, int k, double time,
     double dt, int n_steps, const typename T::shared_state& shared,
@@ -350,7 +350,7 @@ __device__ __forceinline__ void step_particle(
     random::rng_state& rng, const F& done) {
   typename T::internal_state internal{};
   double x[T::n_state_max];
-  if constexpr (has_count_update<T>::value) {
+  if constexpr (COUNTS) {
     const auto c = thread_counts<T>();
     bool ok = !v.deterministic && shared.counts.ready(dt);
     const state_column g{v.state + k, v.stride};
@@ -454,11 +454,11 @@ struct min_blocks_of<T, std::void_t<decltype(T::min_blocks_per_sm)>> {
   __global__ void __launch_bounds__(default_tile_size<T>(),               \
                                     min_blocks_of<T>::value)
 
-// The same for the kernels that step particles as counts (step_particle),
-// which need fewer registers than update() in FP64: a system may declare
-// `step_blocks_per_sm` for them.  The deterministic likelihood's kernels run
-// update(), and lose by such a cap: 4096 SEIR particles, 60 data times,
-// 33.7 ms at 4 blocks per SM, 39.2 at 5.
+// The same for the kernels that step particles as counts (step_particle with
+// COUNTS), which need fewer registers than update() in FP64: a system may
+// declare `step_blocks_per_sm` for them.  Kernels that run update() lose by
+// such a cap: the deterministic likelihood of 4096 SEIR particles, 60 data
+// times, 33.7 ms at 4 blocks per SM, 39.2 at 5.
 template <typename T, typename = void>
 struct step_blocks_of : min_blocks_of<T> {};
 template <typename T>
@@ -466,9 +466,10 @@ struct step_blocks_of<T, std::void_t<decltype(T::step_blocks_per_sm)>> {
   static constexpr int value = T::step_blocks_per_sm;
 };
 
-#define DUST2_STEP_KERNEL(T)                                              \
+#define DUST2_STEP_KERNEL(T, COUNTS)                                      \
   __global__ void __launch_bounds__(default_tile_size<T>(),               \
-                                    step_blocks_of<T>::value)
+                                    COUNTS ? step_blocks_of<T>::value :   \
+                                    min_blocks_of<T>::value)
 
 // The per-particle kernels below run over a layout's run tiles: a block
 // whose particles share one group stages that group's shared state in
@@ -503,9 +504,9 @@ DUST2_PARTICLE_KERNEL(T) k_initial(system_view<T> v, const int* active,
   capture_error(v.errors, v.any_error, k, rng);
 }
 
-template <typename T>
-DUST2_STEP_KERNEL(T) k_run(system_view<T> v, double time, double dt,
-                           int n_steps) {
+template <typename T, bool COUNTS = has_count_update<T>::value>
+DUST2_STEP_KERNEL(T, COUNTS) k_run(system_view<T> v, double time, double dt,
+                                   int n_steps) {
   __shared__ shared_smem<T> sm;
   const tile tl = v.tiles[blockIdx.x];
   const bool mixed = tl.group < 0;
@@ -522,9 +523,9 @@ DUST2_STEP_KERNEL(T) k_run(system_view<T> v, double time, double dt,
   const auto& shared = mixed ? v.shared[g] : sm.shared();
   const zero_every_spec& zero = mixed ? v.zero_every[g] : sm.zero;
   auto rng = load_rng(v.rng, v.stride, k, v.deterministic);
-  step_particle<T>(v, v.state + k, k, time, dt, n_steps, shared, zero,
-                   mixed ? nullptr : sm.zero_steps, rng,
-                   [](const double*, typename T::internal_state&) {});
+  step_particle<T, COUNTS>(v, v.state + k, k, time, dt, n_steps, shared, zero,
+                           mixed ? nullptr : sm.zero_steps, rng,
+                           [](const double*, typename T::internal_state&) {});
   store_rng(v.rng, v.stride, k, rng);
   capture_error(v.errors, v.any_error, k, rng);
 }
@@ -556,12 +557,12 @@ constexpr std::size_t SIM_BUFFER_KEPT = std::size_t(1) << 25;
 // launch per output time, and one to gather its outputs, left the device
 // waiting for the slowest warp each time: 100,003 SIR particles, 60 days of
 // 4 steps, 2.8 ms in 120 launches.
-template <typename T>
-DUST2_STEP_KERNEL(T) k_simulate(system_view<T> v,
-                                const run_segment* segments,
-                                int n_segments, double dt, int n_total,
-                                const int* index_out, int n_out,
-                                double* out) {
+template <typename T, bool COUNTS = has_count_update<T>::value>
+DUST2_STEP_KERNEL(T, COUNTS) k_simulate(system_view<T> v,
+                                        const run_segment* segments,
+                                        int n_segments, double dt,
+                                        int n_total, const int* index_out,
+                                        int n_out, double* out) {
   __shared__ shared_smem<T> sm;
   __shared__ std::conditional_t<segment_steps_fit<T>(), segment_steps,
                                 std::uint64_t[1][1]> zero_steps;
@@ -597,10 +598,10 @@ DUST2_STEP_KERNEL(T) k_simulate(system_view<T> v,
   auto rng = load_rng(v.rng, v.stride, k, v.deterministic);
   for (int i = 0; i < n_segments; ++i) {
     const run_segment seg = segments[i];
-    step_particle<T>(v, v.state + k, k, seg.time, dt, seg.n_steps, shared,
-                     zero, segment_steps_fit<T>() && !mixed ?
-                     zero_steps[i] : nullptr, rng,
-                     [](const double*, typename T::internal_state&) {});
+    step_particle<T, COUNTS>(
+      v, v.state + k, k, seg.time, dt, seg.n_steps, shared, zero,
+      segment_steps_fit<T>() && !mixed ? zero_steps[i] : nullptr, rng,
+      [](const double*, typename T::internal_state&) {});
     double* dst = out + (static_cast<long>(i) * n_total + k) * n_out;
     for (int j = 0; j < n_out; ++j) {
       const int s = index_out == nullptr ? j : index_out[j];
@@ -845,10 +846,12 @@ public:
   void launch_run(double t0, int n_steps) {
     if constexpr (has_update<T>::value && !dust2gpu::is_continuous<T>()) {
       if (n_steps > 0) {
-        k_run<T><<<n_run_tiles(), layout_.tile_size,
-                   count_smem_per_thread<T>() * layout_.tile_size,
-                   stream_>>>(
-          run_view(), t0, dt_, n_steps);
+        with_counts([&](auto counts) {
+          constexpr bool C = decltype(counts)::value;
+          k_run<T, C><<<n_run_tiles(), layout_.tile_size,
+                        C ? count_smem_per_thread<T>() * layout_.tile_size : 0,
+                        stream_>>>(run_view(), t0, dt_, n_steps);
+        });
         DUST2_CUDA(cudaGetLastError());
       }
     } else {
@@ -1101,14 +1104,32 @@ private:
                                cudaMemcpyHostToDevice, stream_));
   }
 
+  // f with true_type where particles may be stepped as counts, which a
+  // deterministic system's never are: its kernels run update() alone, with
+  // the registers that it wants (one SEIR particle, 400 steps: 21.2 ms in
+  // the count kernel's registers).
+  template <typename F>
+  void with_counts(const F& f) {
+    if constexpr (has_count_update<T>::value) {
+      if (!deterministic_) {
+        f(std::true_type{});
+        return;
+      }
+    }
+    f(std::false_type{});
+  }
+
   void launch_simulate(int first, int n, const int* index_dev, int n_out,
                        double* out_dev) {
     if constexpr (has_update<T>::value && !dust2gpu::is_continuous<T>()) {
-      k_simulate<T><<<n_run_tiles(), layout_.tile_size,
-                      count_smem_per_thread<T>() * layout_.tile_size,
-                      stream_>>>(run_view(), segments_.data() + first, n,
-                                 dt_, layout_.n_total, index_dev, n_out,
-                                 out_dev);
+      with_counts([&](auto counts) {
+        constexpr bool C = decltype(counts)::value;
+        k_simulate<T, C><<<n_run_tiles(), layout_.tile_size,
+                           C ? count_smem_per_thread<T>() * layout_.tile_size :
+                           0, stream_>>>(
+          run_view(), segments_.data() + first, n, dt_, layout_.n_total,
+          index_dev, n_out, out_dev);
+      });
       DUST2_CUDA(cudaGetLastError());
     } else {
       throw std::runtime_error("continuous-time system has no update()");

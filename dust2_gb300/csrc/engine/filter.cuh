@@ -215,12 +215,12 @@ __device__ __forceinline__ void step_compare_tile(
     auto rng = load_rng(v.rng, v.stride, k, v.deterministic);
     const int from = src.resampled && f.mode[tl.group] != MODE_KEEP ?
       f.offset[tl.group] + f.idx[k] : k;
-    step_particle<T>(v, src.state + from, k, time, dt, n_steps, sm.shared(),
-                     sm.zero, sm.zero_steps, rng,
-                     [&](const double* x, typename T::internal_state& in) {
-                       logw = T::compare_data(time_compare, x, *d,
-                                              sm.shared(), in, rng);
-                     });
+    step_particle<T, has_count_update<T>::value>(
+      v, src.state + from, k, time, dt, n_steps, sm.shared(), sm.zero,
+      sm.zero_steps, rng,
+      [&](const double* x, typename T::internal_state& in) {
+        logw = T::compare_data(time_compare, x, *d, sm.shared(), in, rng);
+      });
     store_rng(v.rng, v.stride, k, rng);
     capture_error(v.errors, v.any_error, k, rng);
     f.w[k] = logw;
@@ -435,11 +435,10 @@ __global__ void __launch_bounds__(128) k_step_compare_lanes(
 }
 
 template <typename T>
-DUST2_STEP_KERNEL(T) k_step_compare(system_view<T> v, filter_view f,
-                                    step_source src, double time, double dt,
-                                    int n_steps, double time_compare,
-                                    const typename T::data_type* data,
-                                    int n_groups_data) {
+DUST2_STEP_KERNEL(T, has_count_update<T>::value)
+k_step_compare(system_view<T> v, filter_view f, step_source src, double time,
+               double dt, int n_steps, double time_compare,
+               const typename T::data_type* data, int n_groups_data) {
   __shared__ shared_smem<T> sm;
   const tile tl = v.tiles[blockIdx.x];
   if (!f.active[tl.group]) {
@@ -457,7 +456,7 @@ DUST2_STEP_KERNEL(T) k_step_compare(system_view<T> v, filter_view f,
 // groups of very different sizes then share one launch without a block
 // per tile, and a block that finishes early takes the next tile at once.
 template <typename T>
-DUST2_STEP_KERNEL(T) k_step_compare_queue(
+DUST2_STEP_KERNEL(T, has_count_update<T>::value) k_step_compare_queue(
     system_view<T> v, filter_view f, step_source src, double time, double dt,
     int n_steps, double time_compare, const typename T::data_type* data,
     int n_groups_data, int n_tiles, int* next_tile) {

@@ -120,13 +120,11 @@ DUST2_PARTICLE_KERNEL(T) k_served_initial(system_view<T> v,
 // One observation of every running request: the plain filter's
 // step_compare_tile with the session's own interval and data row.
 template <typename T>
-DUST2_STEP_KERNEL(T) k_served_step_compare(system_view<T> v, filter_view f,
-                                           const double* last_state,
-                                           const served_slot* slots,
-                                           const int* obs,
-                                           const obs_step* sched,
-                                           const typename T::data_type* data,
-                                           int* slot_error) {
+DUST2_STEP_KERNEL(T, has_count_update<T>::value)
+k_served_step_compare(system_view<T> v, filter_view f,
+                      const double* last_state, const served_slot* slots,
+                      const int* obs, const obs_step* sched,
+                      const typename T::data_type* data, int* slot_error) {
   __shared__ shared_smem<T> sm;
   const tile tl = v.tiles[blockIdx.x];
   const int g = tl.group;
