@@ -547,6 +547,13 @@ public:
         cudaMemcpyDeviceToHost, copy_stream_));
     }
     DUST2_CUDA(cudaStreamSynchronize(copy_stream_));
+    // After an error the system's time is the start of the last of up to 8
+    // parts of the output times, however many launches there were.
+    const int parts = std::min(n_times, n_sim_chunks);
+    const long last = static_cast<long>(n_times) * (parts - 1) / parts;
+    if (last > 0) {
+      base_.set_time(times[last - 1]);
+    }
     base_.check_errors_after();
     base_.set_time(times[n_times - 1]);
   }

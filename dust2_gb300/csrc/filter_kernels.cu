@@ -580,8 +580,8 @@ __device__ __forceinline__ double chunk_offsets_warp(const double* sums,
 // state is moved before the last barrier is waited for (and again if the
 // group turns out to need the serial algorithm).  One block
 // records the group's sums, generator and log-likelihood, whose logarithm
-// it takes while the others search.  Groups of 1000 particles: 12.0 us an
-// observation (15.2 with four barriers around one block's sums).
+// it takes while the others search.  Groups of 1000 particles: 11.0 us a
+// launch (15.2 with four barriers around one block's sums).
 // Every block of a running group takes both barriers whatever the data, and
 // the third exactly when its flag, the same in every block, is set.
 template <int BLOCK>
