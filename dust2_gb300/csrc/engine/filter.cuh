@@ -235,10 +235,18 @@ __device__ __forceinline__ void step_compare_tile(
 // advance()), and compares its state as it stands, outputs not refreshed
 // (continuous/system.hpp:279-305).  The group reductions are
 // k_step_compare's.
-// (Registers as the solver needs them, 255 at most: the number of warps is
-// not what bounds it.)
-template <typename T>
-__global__ void __launch_bounds__(default_tile_size<T>())
+//
+// The solver wants all 255 registers, with which an SM partition holds two
+// warps.  Between two and three warps of particles per partition the third
+// would then run after the others: with THREE, 168 registers and one-warp
+// blocks let it run beside them.  One group of malaria particles, 10 data
+// times of one step, ms a run at 38,000 / 42,000 / 50,000 / 58,000 / 60,000
+// particles: 255 registers 11.6 / 18.2 / 20.1 / 20.5 / 20.3, 168 registers
+// 13.7 / 15.9 / 17.1 / 17.8 / 21.6 (128 registers and no lazy record, as it
+// once was: 14.0 / 17.3 / 18.2 / 18.9 / 22.4).
+template <typename T, bool THREE>
+__global__ void __launch_bounds__(THREE ? 32 : default_tile_size<T>(),
+                                  THREE ? 12 : 1)
 k_step_compare_mixed(
     system_view<T> v, ode_view o, dopri5::control_dev ctl, filter_view f,
     double time0, double time, double dt, int initialise,
@@ -653,8 +661,16 @@ public:
       constexpr int per_warp = 32 / MIXED_LANES;
       mixed_lanes_ = has_lanes<T>::value && owner_->dt() > 0 &&
         no_resets(sys_->zero_every_specs()) && N <= 3 * per_warp * 4 * n_sms();
+      long warps = 0;
+      for (int n : L.n_particles) {
+        warps += (n + 31) / 32;
+      }
+      mixed_three_ = !mixed_lanes_ && warps > 2 * 4L * n_sms() &&
+        warps <= 3 * 4L * n_sms();
       if (mixed_lanes_) {
         first = step_shape{32, per_warp, false};
+      } else if (mixed_three_) {
+        first = step_shape{32, 0, false};
       }
     }
     set_shape(first);
@@ -1491,7 +1507,8 @@ private:
         }
         if (!mixed_lanes_) {
           launch_after_previous(
-            overlap, k_step_compare_mixed<T>, n_step_tiles_, shape_.block, 0,
+            overlap, mixed_three_ ? k_step_compare_mixed<T, true> :
+            k_step_compare_mixed<T, false>, n_step_tiles_, shape_.block, 0,
             s, v, record, owner_->control_dev(), f, st.t0, st.t_compare,
             owner_->dt(), i == 0 ? 1 : 0, data_.data() + i * n_groups_data_,
             n_groups_data_);
@@ -1672,6 +1689,7 @@ private:
   bool has_run_ = false;
   bool use_graph_ = true;
   bool mixed_lanes_ = false;  // k_step_compare_lanes
+  bool mixed_three_ = false;  // k_step_compare_mixed with three warps
   bool fused_tail_ = false;  // k_tail_cluster instead of separate kernels
   int tail_block_ = 0;       // its block size for these groups (0: none)
   int group_threads_ = 32;   // block size of k_group
