@@ -254,9 +254,15 @@ struct seir_age {
       std::frexp(top, &e);  // top < 2^e
       c.scale[a] = 32 - e;
       c.ok = c.ok && top > 0 && c.scale[a] >= 32 && c.scale[a] <= 62;
-      for (int b = 0; b < n_age && c.ok; ++b) {
-        const double k = std::floor(std::ldexp(row[b], c.scale[a]) + 0.5);
-        c.k[a][b] = static_cast<std::uint32_t>(std::min(k, 4294967295.0));
+      if (!c.ok) {
+        break;
+      }
+      // rounded to nearest; at most 2^32, so cut off there
+      const double unit = std::ldexp(1.0, c.scale[a]);
+      for (int b = 0; b < n_age; ++b) {
+        const auto k = static_cast<std::uint64_t>(row[b] * unit + 0.5);
+        c.k[a][b] = static_cast<std::uint32_t>(
+          std::min<std::uint64_t>(k, 0xffffffffu));
       }
     }
   }
